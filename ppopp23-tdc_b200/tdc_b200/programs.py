@@ -6,12 +6,14 @@ calls run it with one library call.  The modules stay what they are — paramete
 was built from is compared with them on every call, AFTER the launches are issued, so that the comparison costs no latency:
 where something changed (a weight written to or replaced, a submodule exchanged, a hook registered) the nets are dropped and
 the forward runs again.  A network that a net cannot express (an exotic stride, a hook that wants to see a layer) runs
-layer by layer as before."""
+layer by layer.  So does one with a module of another kind in a place that the layer-by-layer forward CALLS (stages, blocks, the
+average pool, the classifier): a net stands for the forwards of the exact classes named in the builders, no subclass's."""
 import math
 import threading
 
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as _module
 
 from . import net as N
 from ._lib import ERR_SHAPE, ERR_SMEM, ERR_UNSUPPORTED, NetConv, TdcError, check, lib
@@ -25,6 +27,18 @@ NCHW_PRECISIONS = ("fp32", "tf32x3", "tf32")     # the layer-by-layer kernels, l
 
 class NotExpressible(Exception):
     """This network or layer is no chain of the launches a net has."""
+
+
+def _exact(module, *kinds):
+    """`module`, if its forward is the one of these classes that a net stands for."""
+    if type(module) not in kinds:
+        raise NotExpressible
+    return module
+
+
+def _average_to_one(pool):
+    if _exact(pool, nn.AdaptiveAvgPool2d).output_size not in (1, (1, 1), [1, 1]):
+        raise NotExpressible
 
 
 # ---- BatchNorm folding -----------------------------------------------------------------------------------------------
@@ -233,10 +247,12 @@ def pool_max(net, m, x, out):
 
 # ---- the networks ----------------------------------------------------------------------------------------------------
 def build_resnet(model, net, precision):
-    from .resnet import TKBottleneck
+    from .resnet import TKBasicBlock, TKBottleneck
+    _average_to_one(model.avgpool)
+    _exact(model.fc, nn.Linear)
     s, b, _ = fold_bn(model.bn1)
-    blocks = [m for layer in (model.layer1, model.layer2, model.layer3, model.layer4) for m in layer]
-    wide = [isinstance(m, TKBottleneck) for m in blocks]
+    blocks = [_exact(m, TKBasicBlock, TKBottleneck) for layer in (model.layer1, model.layer2, model.layer3, model.layer4) for m in _exact(layer, nn.Sequential)]
+    wide = [type(m) is TKBottleneck for m in blocks]
 
     def strided(i):
         return i < len(blocks) and (blocks[i].conv2 if wide[i] else blocks[i].conv1).stride[0] == 2
@@ -272,6 +288,10 @@ def build_resnet(model, net, precision):
 
 def build_vgg(model, net, precision):
     from .resnet import Conv2dB200
+    from .vgg import TKVGG
+    if type(model).forward_features is not TKVGG.forward_features:
+        raise NotExpressible
+    _exact(model.head.fc, nn.Linear)
     mods = list(model.features)
     x, i = None, 0
     B, Cc, H, W = net.shape
@@ -314,7 +334,15 @@ def build_vgg(model, net, precision):
 
 
 def build_densenet(model, net, precision):
-    from .densenet import TKDenseBlock, TKDenseTransition
+    from .densenet import TKDenseBlock, TKDenseLayer, TKDenseNet, TKDenseTransition
+    if type(model).forward_features is not TKDenseNet.forward_features:
+        raise NotExpressible
+    _average_to_one(model.global_pool)
+    _exact(model.classifier, nn.Linear)
+    for name, m in model.features.named_children():
+        if name.startswith(("denseblock", "transition")) and type(_exact(m, TKDenseBlock, TKDenseTransition)) is TKDenseBlock:
+            for layer in m.values():
+                _exact(layer, TKDenseLayer)
     if net.nchw:
         return build_densenet_nchw(model, net, precision)
     f = model.features
@@ -327,7 +355,6 @@ def build_densenet(model, net, precision):
     for m in stages:
         if isinstance(m, TKDenseBlock):
             layers = list(m.values())
-            probe = x if isinstance(x, At) else None
             if buf is None:
                 Hs, Ws = net.shape[2], net.shape[3]
                 H, W = _pooled(f.pool0, -(-Hs // 2)), _pooled(f.pool0, -(-Ws // 2))
@@ -419,13 +446,14 @@ class Nets:
         self.nets, self.lock = {}, threading.Lock()
         self.parts, self.tensors, self.modules, self.mark = [], [], [], None
         if model is not None:
-            self.modules = list(model.modules())[1:]
+            self.modules = list(model.modules())[1:]          # (not the model itself: it holds this object)
             for m in [model] + self.modules:
                 self.parts += [(m._modules, k, c) for k, c in m._modules.items()]
                 for d in (m._parameters, m._buffers):
                     self.parts += [(d, k, None) for k, t in d.items() if t is None]
                     self.tensors += [(d, k) for k, t in d.items() if t is not None and t.dtype.is_floating_point]
             self.blocks = [m for m in self.modules if "precision" in m.__dict__]
+            self.types = [type(m) for m in [model] + self.modules]
             self.mark = self.state()
 
     def __deepcopy__(self, memo):
@@ -437,13 +465,21 @@ class Nets:
     def state(self):
         return [(t._version, t.data_ptr()) for t in [d.get(k) for d, k in self.tensors]]
 
-    def plain(self, precision):
-        """Whether the submodules' own forwards would do what the network says: no hooks, eval mode, one precision."""
-        return not any(m._forward_hooks or m._forward_pre_hooks or m.training for m in self.modules) and all(m.precision == precision for m in self.blocks)
+    def plain(self, model):
+        """Whether the submodules' own forwards would do what the network says: no hooks, eval mode, one precision, no forward of
+        one object's own."""
+        if _module._global_forward_hooks or _module._global_forward_pre_hooks or "forward_features" in model.__dict__:
+            return False
+        for m in self.modules:
+            d = m.__dict__
+            if m._forward_hooks or m._forward_pre_hooks or m.training or "forward" in d or "new_features" in d:
+                return False
+        return all(m.precision == model.precision for m in self.blocks)
 
-    def fresh(self, precision):
+    def fresh(self, model):
         try:
-            return self.mark is not None and all(d.get(k) is c for d, k, c in self.parts) and self.state() == self.mark and self.plain(precision)
+            return self.mark is not None and all(d.get(k) is c for d, k, c in self.parts) and self.types == [type(m) for m in [model] + self.modules] \
+                and self.state() == self.mark and self.plain(model)
         except AttributeError:        # a tensor is gone
             return False
 
@@ -457,9 +493,9 @@ def forward(model, x, build):
         key = (x.shape, x.device.index, model.precision)
         net = cache.nets.get(key)
         if net is None:
-            if not cache.plain(model.precision):
+            if not cache.plain(model):
                 return None
-            if cache.fresh(model.precision):
+            if cache.fresh(model):
                 with cache.lock, _on_device(x.device):
                     net = cache.nets.get(key)
                     if net is None:
@@ -470,7 +506,7 @@ def forward(model, x, build):
             return None
         if net is not None:
             y = net(x)
-            if cache.fresh(model.precision):
+            if cache.fresh(model):
                 return y
         model.__dict__["_nets"] = None
     return None
@@ -483,7 +519,7 @@ def _build(model, x, build):
         net = N.Net(*x.shape, x.device)
         net.nchw = model.precision in NCHW_PRECISIONS
         return build(model, net, model.precision)
-    except NotExpressible:
+    except (NotExpressible, AttributeError, TypeError, IndexError, KeyError):      # (a module without what the builders read: the layers decide)
         return False
     except TdcError as e:
         if e.code in (ERR_SMEM, ERR_UNSUPPORTED, ERR_SHAPE):

@@ -1,0 +1,159 @@
+"""Which networks run as a net of prepared launches, and when a net is made anew: the builders and the cache of programs.py
+on the CPU, with a stand-in for the library's object that records the steps."""
+import types
+
+import pytest
+import torch
+import torch.nn as nn
+
+
+class Steps:
+    """Takes the calls of net.Net and keeps them; running it gives zeros of the output's shape."""
+    made = []
+
+    def __init__(self, B, C, H, W, device):
+        self.shape, self.device, self.nchw, self.steps = (B, C, H, W), device, False, []
+        Steps.made.append(self)
+
+    def _step(self, *what):
+        self.steps.append(what)
+        return len(self.steps)
+
+    def pack(self, kind=0):
+        return self._step("pack", kind)
+
+    def conv(self, src, kind, weight, **kw):
+        return self._step("conv", src, kind, tuple(weight.shape), kw.get("residual", -1))
+
+    def planes(self, *shape):
+        return self._step("planes", *shape)
+
+    def pool(self, src, k, stride, pad=0, **kw):
+        return self._step("pool", src, k, stride, pad)
+
+    def head(self, src, *a, **kw):
+        return self._step("head", src)
+
+    def finish(self, out_shape):
+        self.out_shape = tuple(out_shape)
+        return self
+
+    def __call__(self, x):
+        return torch.zeros(self.out_shape)
+
+
+@pytest.fixture
+def P(built, monkeypatch):
+    from tdc_b200 import programs
+    Steps.made = []
+    monkeypatch.setattr(programs.N, "Net", Steps)
+    monkeypatch.setattr(programs, "_estimate", lambda *a, **kw: 1.0)
+    monkeypatch.setattr(programs, "_pooled_estimates", lambda *a, **kw: (2.0, 1.0))
+    monkeypatch.setattr(programs, "fold_bn", lambda bn: (bn.running_var, bn.running_mean, bn.running_var[:2]))
+    return programs
+
+
+def nets(T):
+    return {"resnet18": (T.tkc_resnet18, "build_resnet", 64), "resnet50": (T.tkc_resnet50, "build_resnet", 64), "vgg": (lambda **k: T.TKVGG(cfg=[8, "M", 16], **k), "build_vgg", 16),
+            "densenet": (lambda **k: T.TKDenseNet(8, (2, 2), num_classes=10, **k), "build_densenet", 64)}
+
+
+def make(P, name, **kw):
+    """(model, a call that gives its net's output or None where it has to run layer by layer)"""
+    import tdc_b200 as T
+    from tdc_b200 import densenet, vgg  # noqa: F401
+    T = types.SimpleNamespace(tkc_resnet18=T.tkc_resnet18, tkc_resnet50=T.tkc_resnet50, TKVGG=vgg.TKVGG, TKDenseNet=densenet.TKDenseNet)
+    ctor, build, size = nets(T)[name]
+    model = ctor(precision="auto", **kw).eval()
+    return model, caller(P, model, build, size)
+
+
+def caller(P, model, build, size, channels=3):
+    def call(B=1, H=size, W=size, channels=channels):
+        with torch.no_grad():
+            return P.forward(model, torch.zeros(B, channels, H, W), getattr(P, build))
+    return call
+
+
+NAMES = ("resnet18", "resnet50", "vgg", "densenet")
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_the_stock_networks_are_nets(P, name):
+    model, call = make(P, name)
+    assert call() is not None and len(Steps.made) == 1
+    assert call() is not None and len(Steps.made) == 1
+
+
+class Scaled(nn.Linear):
+    def forward(self, x):
+        return 2 * super().forward(x)
+
+
+def with_own_forward(block):
+    class Own(block):
+        def forward(self, x):
+            return 2 * super().forward(x)
+    return Own
+
+
+REPLACED = {
+    "avgpool": ("resnet18", lambda m: setattr(m, "avgpool", nn.AdaptiveMaxPool2d(1))),
+    "maxpool": ("resnet18", lambda m: setattr(m, "maxpool", nn.AvgPool2d(2))),
+    "avgpool's size": ("resnet18", lambda m: setattr(m, "avgpool", nn.AdaptiveAvgPool2d(2))),
+    "stage": ("resnet18", lambda m: setattr(m, "layer4", nn.Identity())),
+    "stage with its own forward": ("resnet50", lambda m: setattr(m.layer2, "__class__", type("S", (nn.Sequential,), {"forward": lambda self, x: x}))),
+    "block with its own forward": ("resnet18", lambda m: setattr(m.layer1[0], "__class__", with_own_forward(type(m.layer1[0])))),
+    "bottleneck with its own forward": ("resnet50", lambda m: setattr(m.layer1[0], "__class__", with_own_forward(type(m.layer1[0])))),
+    "a forward of one block": ("resnet18", lambda m: setattr(m.layer1[0], "forward", lambda x: x)),
+    "global_pool": ("densenet", lambda m: setattr(m, "global_pool", nn.AdaptiveMaxPool2d(1))),
+    "dense block with its own forward": ("densenet", lambda m: setattr(m.features.denseblock1, "__class__", with_own_forward(type(m.features.denseblock1)))),
+    "transition with its own forward": ("densenet", lambda m: setattr(m.features.transition1, "__class__", with_own_forward(type(m.features.transition1)))),
+    "dense layer of another kind": ("densenet", lambda m: setattr(m.features.denseblock1.denselayer1, "__class__",
+                                                                 type("L", (type(m.features.denseblock1.denselayer1),), {"new_features": lambda self, p, q: p}))),
+    "new features of one layer": ("densenet", lambda m: setattr(m.features.denseblock1.denselayer1, "new_features", lambda p, q: p)),
+    "features of a subclass": ("densenet", lambda m: setattr(m, "__class__", type("D", (type(m),), {"forward_features": lambda self, x: x}))),
+    "features of a VGG subclass": ("vgg", lambda m: setattr(m, "__class__", type("V", (type(m),), {"forward_features": lambda self, x: x}))),
+}
+
+
+@pytest.mark.parametrize("what", sorted(REPLACED))
+@pytest.mark.parametrize("before", [True, False])
+def test_a_module_that_does_something_else_is_called(P, what, before):
+    """What the layer-by-layer forward calls — stages, blocks, the average pool — a net may only replace where it is the module
+    whose arithmetic the net has; replaced before the first call and after it."""
+    name, change = REPLACED[what]
+    model, call = make(P, name)
+    if not before:
+        assert call() is not None
+    change(model)
+    assert call() is None and call() is None
+
+
+HEADS = {"resnet18": "fc", "vgg": "head.fc", "densenet": "classifier"}
+
+
+@pytest.mark.parametrize("name", sorted(HEADS))
+@pytest.mark.parametrize("head", ["identity", "chain", "subclass"])
+@pytest.mark.parametrize("before", [True, False])
+def test_any_classifier_is_called(P, name, head, before):
+    model, call = make(P, name)
+    if not before:
+        assert call() is not None
+    owner, _, leaf = HEADS[name].rpartition(".")
+    n = model.get_submodule(HEADS[name]).in_features
+    own = {"identity": nn.Identity, "chain": lambda: nn.Sequential(nn.Linear(n, 7)), "subclass": lambda: Scaled(n, 7)}[head]().eval()
+    setattr(model.get_submodule(owner), leaf, own)
+    assert call() is None
+
+
+def test_hooks_on_every_module(P):
+    """torch.nn.modules.module.register_module_forward_hook: every module has to be called."""
+    model, call = make(P, "resnet18")
+    assert call() is not None
+    h = nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert call() is None
+    finally:
+        h.remove()
+    assert call() is not None
