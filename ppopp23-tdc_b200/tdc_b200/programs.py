@@ -45,7 +45,7 @@ def _average_to_one(pool):
 def fold_bn(bn):
     """(scale, shift, {max |scale|, max |shift|}) of an inference BatchNorm on the GPU, kept on the module until one of its
     tensors changes."""
-    key = N._key(bn.running_var, bn.running_mean, bn.weight, bn.bias)
+    key = (bn.eps,) + N._key(bn.running_var, bn.running_mean, bn.weight, bn.bias)
     hit = bn.__dict__.get("_tdc_fold")
     if hit is None or hit[0] != key:
         n, dev = bn.running_var.numel(), bn.running_var.device
@@ -439,12 +439,16 @@ def _pooled(m, n):
 
 # ---- the cache on a model ----------------------------------------------------------------------------------------------
 class Nets:
-    """The nets of one model by input shape, and what they were built from."""
+    """The nets of one model by input shape, and what they were built from: the modules and their classes, the tensors, the
+    keys of every table of children, parameters and buffers, and the plain attributes the builders read."""
+    READ = ("stride", "padding", "dilation", "groups", "kernel_size", "ceil_mode", "output_size", "eps", "in_channels", "out_channels", "in_rank", "out_rank", "rank",
+            "num_features", "num_input_features", "num_output_features", "growth_rate", "in_features", "out_features", "downsample")
     MOST = 16                     # shapes kept: the oldest goes first
 
     def __init__(self, model=None):
         self.nets, self.lock = {}, threading.Lock()
         self.parts, self.tensors, self.modules, self.mark = [], [], [], None
+        self.orders, self.sizes, self.lengths, self.read, self.values = [], [], [], [], []
         if model is not None:
             self.modules = list(model.modules())[1:]          # (not the model itself: it holds this object)
             for m in [model] + self.modules:
@@ -452,6 +456,12 @@ class Nets:
                 for d in (m._parameters, m._buffers):
                     self.parts += [(d, k, None) for k, t in d.items() if t is None]
                     self.tensors += [(d, k) for k, t in d.items() if t is not None and t.dtype.is_floating_point]
+                if m._modules:
+                    self.orders.append((m._modules, list(m._modules)))
+                self.sizes += [m._modules, m._parameters, m._buffers]
+                self.read += [(m.__dict__, k) for k in self.READ if k in m.__dict__]
+            self.lengths = [len(d) for d in self.sizes]
+            self.values = [d[k] for d, k in self.read]
             self.blocks = [m for m in self.modules if "precision" in m.__dict__]
             self.types = [type(m) for m in [model] + self.modules]
             self.mark = self.state()
@@ -476,39 +486,35 @@ class Nets:
                 return False
         return all(m.precision == model.precision for m in self.blocks)
 
-    def fresh(self, model):
+    def current(self, model):
+        """Whether the model still is what the nets were built from."""
         try:
             return self.mark is not None and all(d.get(k) is c for d, k, c in self.parts) and self.types == [type(m) for m in [model] + self.modules] \
-                and self.state() == self.mark and self.plain(model)
+                and self.lengths == [len(d) for d in self.sizes] and all(list(d) == keys for d, keys in self.orders) \
+                and self.values == [d.get(k) for d, k in self.read] and self.state() == self.mark
         except AttributeError:        # a tensor is gone
             return False
 
 
 def forward(model, x, build):
     """The model's output for x through its net, or None where it has to run layer by layer."""
-    for _ in range(2):
+    for _ in range(4):                # (found out of date, built, run)
         cache = model.__dict__.get("_nets")
         if cache is None or cache.mark is None:
             cache = model.__dict__["_nets"] = Nets(model)
         key = (x.shape, x.device.index, model.precision)
         net = cache.nets.get(key)
-        if net is None:
-            if not cache.plain(model):
-                return None
-            if cache.fresh(model):
-                with cache.lock, _on_device(x.device):
-                    net = cache.nets.get(key)
-                    if net is None:
-                        net = cache.nets[key] = _build(model, x, build)
-                        while len(cache.nets) > Nets.MOST:
-                            cache.nets.pop(next(iter(cache.nets)))
-        if net is False:
-            return None
-        if net is not None:
-            y = net(x)
-            if cache.fresh(model):
-                return y
-        model.__dict__["_nets"] = None
+        y = net(x) if net else None
+        if not cache.current(model):
+            model.__dict__["_nets"] = None
+        elif net or net is False or not cache.plain(model):
+            return y if cache.plain(model) else None
+        else:
+            with cache.lock, _on_device(x.device):
+                if key not in cache.nets:
+                    cache.nets[key] = _build(model, x, build)
+                    while len(cache.nets) > Nets.MOST:
+                        cache.nets.pop(next(iter(cache.nets)))
     return None
 
 
@@ -552,7 +558,7 @@ def layer(module, x):
         cache = module.__dict__["_layer_net"] = _LayerNet()
         cache.mark = mark
         cache.keep = [t.detach() for t in (first, core, last, bias) if t is not None]      # the mark holds their addresses
-    key = (x.shape, module.precision, x.device.index)
+    key = (x.shape, module.precision, x.device.index, module.stride, module.padding, module.dilation, module.groups)
     net = cache.nets.get(key)
     if net is None:
         while len(cache.nets) >= Nets.MOST:

@@ -157,3 +157,75 @@ def test_hooks_on_every_module(P):
     finally:
         h.remove()
     assert call() is not None
+
+
+def appended_block(m):
+    import tdc_b200.resnet as R
+    m.layer1.append(R.TKBasicBlock(64, 64, stage=1, id=1, hp_dict=R.HalfRanks()).eval())
+    m.layer1[-1].precision = m.precision
+
+
+CHANGED = {
+    "appended block": ("resnet18", appended_block),
+    "order of the children": ("resnet18", lambda m: m.layer1._modules.move_to_end("0") if hasattr(m.layer1._modules, "move_to_end")
+                              else m.layer1._modules.__setitem__("0", m.layer1._modules.pop("0"))),
+    "a new child": ("vgg", lambda m: m.features.add_module("9", nn.MaxPool2d(2).eval())),
+    "eps": ("resnet50", lambda m: setattr(m.layer3[0].bn2, "eps", 0.5)),
+    "pool geometry": ("resnet18", lambda m: setattr(m.maxpool, "kernel_size", 5) or setattr(m.maxpool, "padding", 2)),
+    "stride of a convolution": ("resnet18", lambda m: setattr(m.layer2[0].conv1, "stride", (1, 1)) or setattr(m.layer2[0].downsample[0], "stride", (1, 1))),
+    "a shortcut taken out": ("resnet18", lambda m: setattr(m.layer1[0], "downsample", None) or setattr(m.layer1[1], "downsample", nn.Sequential(nn.Conv2d(64, 64, 1), nn.BatchNorm2d(64)).eval())),
+    "a bias": ("densenet", lambda m: m.features.conv0.register_parameter("bias", nn.Parameter(torch.zeros(16)))),
+    "a weight": ("vgg", lambda m: m.features[0].weight.mul_(2)),
+}
+
+
+@pytest.mark.parametrize("what", sorted(CHANGED))
+def test_what_a_net_was_built_from_is_compared(P, what):
+    """Structure, plain attributes and tensors: each of these changes what the layer-by-layer forward computes."""
+    name, change = CHANGED[what]
+    model, call = make(P, name)
+    assert call() is not None and call() is not None and len(Steps.made) == 1
+    with torch.no_grad():
+        change(model)
+    call()
+    assert len(Steps.made) == 2
+    call()
+    assert len(Steps.made) == 2
+
+
+def test_a_network_that_becomes_expressible_is_a_net_again(P):
+    model, call = make(P, "resnet18")
+    pool, model.avgpool = model.avgpool, nn.AdaptiveMaxPool2d(1)
+    assert call() is None and call() is None
+    model.avgpool = pool
+    assert call() is not None
+
+
+def test_folded_batchnorm_notices_eps(built, monkeypatch):
+    """The fold is kept on the module until one of its tensors, or eps, changes."""
+    from tdc_b200 import programs
+    asked = []
+    monkeypatch.setattr(programs, "lib", types.SimpleNamespace(tdc_net_fold_bn=lambda *a: asked.append(a[4]) or 0))
+    monkeypatch.setattr(programs, "_stream", lambda: 0)
+    bn = nn.BatchNorm2d(8).eval()
+    programs.fold_bn(bn), programs.fold_bn(bn)
+    bn.eps = 0.25
+    programs.fold_bn(bn)
+    assert asked == [1e-5, 0.25]
+
+
+def test_tucker_module_notices_its_geometry(built, monkeypatch):
+    """A Tucker module's net is for one stride and padding."""
+    import tdc_b200 as T
+    from tdc_b200 import programs
+
+    class HP:
+        ranks = {"l": [8, 8]}
+    made = []
+    monkeypatch.setattr(programs, "_build_layer", lambda m, x: made.append((m.stride, m.padding)) or False)
+    m = T.TKConv2dC_B200(16, 16, 3, padding=1, hp_dict=HP, name="l")
+    x = torch.zeros(1, 16, 8, 8)
+    for stride, padding in (((1, 1), (1, 1)), ((1, 1), (1, 1)), ((2, 2), (1, 1)), ((2, 2), (0, 0))):
+        m.stride, m.padding = stride, padding
+        assert programs.layer(m, x) is None
+    assert made == [((1, 1), (1, 1)), ((2, 2), (1, 1)), ((2, 2), (0, 0))]
