@@ -209,7 +209,7 @@ __device__ __forceinline__ void store(const Args& a, const Where& w, int k0, f2 
         for (int k = 0; k < W; ++k) {
             float p, q;
             f2_get(v[k], p, q);
-            v[k] = f2_of(fmaxf(p, 0.f), fmaxf(q, 0.f));
+            v[k] = f2_of(max_nan(p, 0.f), max_nan(q, 0.f));
         }
     }
     float m = ymax;
@@ -372,7 +372,7 @@ __device__ __forceinline__ void pool_columns(const f2 (&p)[8], int odd, float (&
         f2_get(p[k + 4], b0, b1);
         const float k0 = odd ? b0 : a0, k1 = odd ? b1 : a1;
         const float r0 = __shfl_xor_sync(0xffffffffu, odd ? a0 : b0, 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? a1 : b1, 1);
-        m[2 * k] = fmaxf(k0, r0); m[2 * k + 1] = fmaxf(k1, r1);
+        m[2 * k] = max_nan(k0, r0); m[2 * k + 1] = max_nan(k1, r1);
         next[2 * k] = odd ? k0 : r0; next[2 * k + 1] = odd ? k1 : r1;
     }
 }
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) conv_pk_kernel(const __grid_con
                             if (!real) v[k] = 0ull;
                             f2_get(v[k], a0, a1);
                             f2_get(p[k], b0, b1);
-                            p[k] = f2_of(fmaxf(a0, b0), fmaxf(a1, b1));
+                            p[k] = f2_of(max_nan(a0, b0), max_nan(a1, b1));
                         }
                     };
                     if (act) {
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) conv_pk_kernel(const __grid_con
                             for (int k = 0; k < 8; ++k) {
                                 float b0, b1;
                                 f2_get(v[k], b0, b1);
-                                above[k] = f2_of(fmaxf(b0, 0.f), fmaxf(b1, 0.f));
+                                above[k] = f2_of(max_nan(b0, 0.f), max_nan(b1, 0.f));
                             }
                         }
                     }
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) conv_pk_kernel(const __grid_con
                             for (int k = 0; k < 8; ++k) next[k] = q > 0 ? left[k] : 0.f;
                         }
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) m[k] = fmaxf(m[k], next[k]);
+                        for (int k = 0; k < 8; ++k) m[k] = max_nan(m[k], next[k]);
                     }
                     if (k0 >= k_end) continue;
                     f2 out[4];

@@ -385,7 +385,7 @@ __device__ __forceinline__ void store_chunk(const Args& a, const uint32_t (&r)[W
     }
     if (a.relu) {
 #pragma unroll
-        for (int k = 0; k < W; ++k) v[k] = fmaxf(v[k], 0.f);
+        for (int k = 0; k < W; ++k) v[k] = max_nan(v[k], 0.f);
     }
     if (vmax && live) {                              // largest stored magnitude (as a bit pattern: a NaN must not get lost)
         unsigned int m = __float_as_uint(*vmax);

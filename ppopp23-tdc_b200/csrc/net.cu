@@ -248,7 +248,7 @@ int tdc_net_pack(tdc_net* n, int kind, int* out) {
     Tensor& t = n->tensors[id];
     PackArgs a{};
     a.B = n->B; a.C = n->C; a.H = n->H; a.W = n->W;
-    a.groups = t.groups; a.front = space_front(s); a.d = s; a.y_plane = tdc_net::pk_plane(t);
+    a.groups = t.groups; a.front = space_front(s); a.d = s; a.y_plane = tdc_net::pk_plane(t); a.status = n->f.status;
     const unsigned grid = blocks_for(items, n->f);
     t.slots = (int)grid;
     const void* fn = kind == PACK_SAME ? (const void*)&pack_kernel<PACK_SAME> : kind == PACK_SPLIT ? (const void*)&pack_kernel<PACK_SPLIT>

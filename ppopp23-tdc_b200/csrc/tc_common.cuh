@@ -43,6 +43,14 @@ __host__ __device__ __forceinline__ float range_scale(float m, int target = 14) 
     return ldexpf(1.f, k);
 }
 
+// The larger of two values; a NaN wins.  fmaxf drops it: an input that left fp16's range arrives in an epilogue as inf - inf, and a
+// ReLU or a maximum by fmaxf would make it a zero that nothing reports.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {

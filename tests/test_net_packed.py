@@ -2,11 +2,15 @@
 
 The bar is that of a single layer with fp32-level operands (FP32_TOL): both operands are split into two fp16 parts that carry
 22 bits, products of the two lo parts (2^-22) are left out, sums are fp32."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 import torch.nn.functional as F
 
-from helpers import FP32_TOL
+from helpers import FP32_TOL, ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -268,3 +272,63 @@ def test_nchw_nets_equal_the_layers(N, net, precision):
         ref = m(x)                               # a hook makes the network run layer by layer
         h.remove()
     assert rel(y, ref.double()) <= FP32_TOL
+
+
+OVERFLOW = """
+import sys
+for p in sys.argv[1:3]:
+    sys.path.insert(0, p)
+import torch
+import tdc_b200 as T
+from tdc_b200 import net as N, tc
+kind, R, pack, pool, tile, C, K, H, W = eval(sys.argv[3])
+g = torch.Generator().manual_seed(1)
+x = torch.randn(2, C, H, W, generator=g).cuda()
+w = torch.randn(K, C, R, R, generator=g).cuda()
+
+
+def run(x):
+    net = N.Net(*x.shape, x.device)
+    t = net.conv(net.pack(pack), kind, w, relu=True, out=N.PLANES if pool else N.NCHW, pool=pool, tile=tile)
+    if pool:
+        net.head(t, torch.eye(K, device="cuda"), None)
+        return net.finish((2, K))(x)
+    return net.finish((2, K, H, W))(x)
+
+
+assert bool(run(x).isfinite().all()) and tc.status() == 0
+x[1, 0, H // 2, W // 2] = 1e5 * float(x.abs().max())
+y = run(x)
+assert bool(y[0].isfinite().all()) and not bool(y[1].isfinite().all()), y
+assert tc.status() == 2
+conv = T.TcConv(torch.randn(K, C, 3, 3, generator=g).cuda(), mode=4)
+conv.packed = False
+assert not bool(conv(x, relu=True)[1].isfinite().all())
+"""
+
+
+@pytest.mark.parametrize("case", [(1, 3, 0, 0, (64, 2, 0), 16, 64, 20, 20), (1, 3, 0, 0, (32, 1, 4), 64, 40, 12, 12), (0, 1, 0, 0, (32, 1, 1), 16, 32, 12, 12),
+                                  (1, 3, 0, 2, (64, 2, 0), 16, 64, 20, 20), (3, 7, 2, 3, (64, 2, 0), 3, 64, 40, 40), (4, 3, 3, 0, (64, 1, 0), 3, 64, 40, 40)])
+def test_overflow_is_reported_behind_relu_and_pooling(N, case):
+    """A value beyond 256 times the sampled maximum: the outputs that read it are not finite, ReLU and maxima included, and the status
+    word says 2 (in a process of its own, because the word keeps its first report)."""
+    r = subprocess.run([sys.executable, "-c", OVERFLOW, os.path.join(ROOT, "ppopp23-tdc_b200"), ROOT, repr(case)], capture_output=True, text=True,
+                       env=dict(os.environ, TDC_TC_TUNING="0"), timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("B,C,H,W", [(16, 3, 224, 224), (2, 16, 12, 125)])
+def test_range_sample_is_spread(N, B, C, H, W):
+    """Values at a fixed distance would all lie in the first columns of a batch of 16 images (and in the first image of a small batch),
+    which are a thousandth of the rest here: the sample has to see the others."""
+    from tdc_b200 import tc
+    x = torch.randn(B, C, H, W, generator=torch.Generator().manual_seed(1))
+    x[:, :, :, 0] *= 1e-3
+    if B == 2:
+        x[0] *= 1e-3
+    x = x.cuda()
+    w = (torch.randn(8, C, 3, 3, generator=torch.Generator().manual_seed(2)) * 0.1).cuda()
+    net = N.Net(B, C, H, W, x.device)
+    net.conv(net.pack(), N.CONV3x3, w, relu=True, out=N.NCHW)
+    y = net.finish((B, 8, H, W))(x)
+    assert rel(y, F.conv2d(x.double(), w.double(), None, 1, 1).relu()) <= FP32_TOL and tc.status() == 0
