@@ -10,7 +10,7 @@ import ctypes as C
 import torch
 
 from . import _lib
-from ._lib import NetConv, NetNchw, NetPool, check, lib
+from ._lib import ERR_SHAPE, NetConv, NetNchw, NetPool, TdcError, check, lib
 from .ops import _dev_f32, _on_device, _stream
 
 PACK, PACK_SPLIT, PACK_S2D, PACK_ROWS = range(4)
@@ -39,6 +39,7 @@ class Net:
         self.shape = (B, Cc, H, W)
         self._h = C.c_void_p()
         self._keep = []                 # everything the launches point to
+        self._channels = {-1: Cc}       # tensor -> its channels (-1: the input)
         self.nchw = False               # which steps the network builders take (programs.py)
         self.clocks = 0.0
         with _on_device(device):
@@ -52,12 +53,27 @@ class Net:
     def pack(self, kind=PACK):
         out = C.c_int()
         check(lib.tdc_net_pack(self._h, kind, C.byref(out)))
-        return out.value
+        return self._made(out.value, self.shape[1] * {PACK_S2D: 4, PACK_ROWS: 3}.get(kind, 1))
+
+    def _made(self, tensor, channels):
+        self._channels[tensor] = channels
+        return tensor
+
+    @staticmethod
+    def _per_channel(channels, *vectors):
+        """The launches read one value per channel behind these pointers."""
+        for v in vectors:
+            if v is not None and v.numel() != channels:
+                raise TdcError(ERR_SHAPE, "%d values for %d channels" % (v.numel(), channels))
 
     def conv(self, src, kind, weight, scale=None, bias=None, relu=False, residual=-1, out=PACKED, split=False, into=-1, into_c=0,
              owner=None, name=None, unbiased=True, tile=None, pool=0):
         """`weight`: [K][C][R][R] tensor.  With an `owner` module the prepared filter is kept there under `name`."""
         K, Cc = weight.shape[:2]
+        # (the prepared filter's size follows from the tensor, its contents from the weight)
+        if Cc * {CONV7x7_S2: 4, CONV3x3_ROWS: 3}.get(kind, 1) != self._channels.get(src, -1):
+            raise TdcError(ERR_SHAPE, "a filter of %d channels on tensor %d of %s" % (Cc, src, self._channels.get(src)))
+        self._per_channel(K, scale, bias)
         d = NetConv()
         d.kind, d.K, d.relu, d.residual, d.out, d.out_split, d.into, d.into_c, d.unbiased = kind, K, int(relu), residual, out, int(split), into, into_c, int(unbiased)
         d.pool = pool
@@ -72,7 +88,7 @@ class Net:
         self._keep += [flt, scale, bias]
         t = C.c_int()
         check(lib.tdc_net_add_conv(self._h, src, C.byref(d), C.byref(t)))
-        return t.value
+        return t.value if into >= 0 or out == NCHW else self._made(t.value, K)
 
     def _filter(self, kind, weight, nt, nbytes, scale, bias, owner, name):
         store = owner.__dict__.setdefault("_net_filters", {}) if owner is not None else {}
@@ -90,9 +106,11 @@ class Net:
     def planes(self, B, Cc, H, W):
         t = C.c_int()
         check(lib.tdc_net_planes(self._h, B, Cc, H, W, C.byref(t)))
-        return t.value
+        return self._made(t.value, Cc)
 
     def pool(self, src, k, stride, pad=0, out=PACKED, scale=None, shift=None, bound=None, channels=0, into=-1):
+        channels_out = channels or self._channels.get(src, -1)
+        self._per_channel(channels_out, scale, shift)
         d = NetPool()
         d.k, d.stride, d.pad, d.channels, d.out, d.into = k, stride, pad, channels, out, into
         for n, t in (("scale", scale), ("shift", shift), ("bound", bound)):
@@ -100,10 +118,11 @@ class Net:
         self._keep += [scale, shift, bound]
         t = C.c_int()
         check(lib.tdc_net_pool(self._h, src, C.byref(d), C.byref(t)))
-        return t.value
+        return t.value if into >= 0 else self._made(t.value, channels_out)
 
     # -- NCHW steps (source -1: the input) ----------------------------------------------------------------------------
     def nchw_conv(self, src, K, R, stride, pad, flt, scale=None, bias=None, residual=-1, relu=False, plan=None, flags=0, to_y=False):
+        self._per_channel(K, scale, bias)
         d = NetNchw()
         d.K, d.R, d.S, d.stride, d.pad, d.flags, d.residual, d.relu = K, R, R, stride, pad, flags, residual, int(relu)
         d.to_y = int(to_y)
@@ -114,27 +133,31 @@ class Net:
         self._keep += [flt, scale, bias]
         t = C.c_int()
         check(lib.tdc_net_nchw_conv(self._h, src, C.byref(d), C.byref(t)))
-        return t.value
+        return t.value if to_y else self._made(t.value, K)
 
     def nchw_pool(self, src, k, stride, pad, mode):
         t = C.c_int()
         check(lib.tdc_net_nchw_pool(self._h, src, k, stride, pad, mode, C.byref(t)))
-        return t.value
+        return self._made(t.value, self._channels.get(src, -1))
 
     def nchw_buffer(self, Cc, H, W):
         t = C.c_int()
         check(lib.tdc_net_nchw_buffer(self._h, Cc, H, W, C.byref(t)))
-        return t.value
+        return self._made(t.value, Cc)
 
     def nchw_affine(self, src, scale=None, shift=None, relu=False, channels=0, into=-1, into_c=0):
+        channels_out = channels or self._channels.get(src, -1)
+        self._per_channel(channels_out, scale, shift)
         self._keep += [scale, shift]
         t = C.c_int()
         check(lib.tdc_net_nchw_affine(self._h, src, channels, scale.data_ptr() if scale is not None else None, shift.data_ptr() if shift is not None else None,
                                       int(relu), into, into_c, C.byref(t)))
-        return t.value
+        return t.value if into >= 0 else self._made(t.value, channels_out)
 
     def head(self, src, weight, bias, scale=None, shift=None):
         weight, bias = weight.detach(), bias.detach() if bias is not None else None      # (aliases: the launches read this memory)
+        self._per_channel(self._channels.get(src, -1), weight[0], scale, shift)
+        self._per_channel(weight.shape[0], bias)
         self._keep += [weight, bias, scale, shift]
         check(lib.tdc_net_head(self._h, src, scale.data_ptr() if scale is not None else None, shift.data_ptr() if shift is not None else None,
                                _dev_f32(weight, "weight"), bias.data_ptr() if bias is not None else None, weight.shape[0]))

@@ -122,6 +122,8 @@ def conv(net, module, x, scale, shift, relu, precision, residual=-1, out=N.PACKE
     pooling = _pool_of(pool) if pool is not None else 0
 
     def step(src, kind, weight, name, last, K):
+        if tuple(weight.shape[:2]) != (K, src.C) or weight.shape[2] != weight.shape[3]:
+            raise NotExpressible
         stride = 2 if kind in (N.CONV3x3_S2, N.CONV1x1_S2) else 1
         opts = end if last else {}
         if last and pool is not None:
@@ -221,9 +223,9 @@ def stem7(net, module, scale, shift, pool, out, precision):
     if tuple(module.kernel_size) != (7, 7) or tuple(module.stride) != (2, 2) or tuple(module.padding) != (3, 3) or tuple(module.dilation) != (1, 1) or module.groups != 1:
         raise NotExpressible
     B, Cc, H, W = net.shape
-    if Cc != module.in_channels:
+    if Cc != module.weight.shape[1]:
         raise NotExpressible
-    t, K, H, W = net.pack(N.PACK_S2D), module.out_channels, -(-H // 2), -(-W // 2)
+    t, K, H, W = net.pack(N.PACK_S2D), module.weight.shape[0], -(-H // 2), -(-W // 2)
     opts = dict(scale=scale, bias=_with_bias(module, scale, shift), relu=True, owner=module, name="weight")
     pooling = _pool_of(pool)
     if pooling:
@@ -318,8 +320,10 @@ def build_vgg(model, net, precision):
             x = At(-1, Cc, H, W)
         elif x is None:
             if type(m) is Conv2dB200 and 3 * Cc <= 16 and _square(m, 3) == 1:
+                if m.weight.shape[1] != Cc:
+                    raise NotExpressible
                 t = net.conv(net.pack(N.PACK_ROWS), N.CONV3x3_ROWS, m.weight, scale=scale, bias=_with_bias(m, scale, shift), relu=relu, out=out, owner=m, name="weight")
-                x = At(t, m.out_channels, H, W)
+                x = At(t, m.weight.shape[0], H, W)
                 continue
             x = At(net.pack(N.PACK), Cc, H, W)
         pool = mods[i] if i < len(mods) and isinstance(mods[i], nn.MaxPool2d) and not net.nchw else None

@@ -229,3 +229,27 @@ def test_tucker_module_notices_its_geometry(built, monkeypatch):
         m.stride, m.padding = stride, padding
         assert programs.layer(m, x) is None
     assert made == [((1, 1), (1, 1)), ((2, 2), (1, 1)), ((2, 2), (0, 0))]
+
+
+@pytest.mark.parametrize("name,channels", [("resnet18", 1), ("vgg", 1), ("vgg", 4), ("vgg", 20), ("densenet", 1)])
+def test_input_of_other_channels_is_left_to_the_layers(P, name, channels):
+    """(whose checks refuse it)"""
+    model, call = make(P, name)
+    assert call(channels=channels) is None
+
+
+def test_filters_and_vectors_match_their_tensor(built):
+    """The launches read the sizes of the tensor behind the pointers of filter, scale, bias and classifier: a mismatch is refused
+    before the library is asked."""
+    from tdc_b200 import TdcError, net as N
+    n = object.__new__(N.Net)
+    n._h, n._keep, n._channels, n.clocks, n.shape = None, [], {-1: 16, 0: 16}, 0.0, (1, 16, 8, 8)
+    ok, w = torch.zeros(8), torch.zeros(8, 16, 1, 1)
+    for call in (lambda: n.conv(0, N.CONV1x1, torch.zeros(8, 17, 1, 1)), lambda: n.conv(0, N.CONV3x3_ROWS, torch.zeros(8, 16, 3, 3)), lambda: n.conv(0, N.CONV7x7_S2, torch.zeros(8, 5, 7, 7)),
+                 lambda: n.conv(1, N.CONV1x1, w), lambda: n.conv(0, N.CONV1x1, w, torch.zeros(7), ok), lambda: n.conv(0, N.CONV1x1, w, ok, torch.zeros(9)),
+                 lambda: n.pool(0, 1, 1, scale=ok, shift=ok, bound=ok), lambda: n.pool(0, 1, 1, scale=ok, shift=ok, bound=ok, channels=4),
+                 lambda: n.nchw_conv(-1, 8, 1, 1, 0, w, scale=torch.zeros(16)), lambda: n.nchw_affine(-1, ok, ok), lambda: n.head(0, torch.zeros(10, 17), None),
+                 lambda: n.head(0, torch.zeros(10, 16), torch.zeros(9))):
+        with pytest.raises(TdcError) as e:
+            call()
+        assert e.value.code == 2          # TDC_ERR_SHAPE
