@@ -46,8 +46,10 @@ def channel_last(owner, name, w):
     key = (w._version, w.data_ptr())
     hit = store.get(name)
     if hit is None or hit[0] != key:
-        w = w.detach().contiguous()
-        hit = store[name] = (key, ops.permute_weights(w), w)      # (the filter itself too: its address is the key)
+        from .net import building
+        with building(w.device):
+            w = w.detach().contiguous()
+            hit = store[name] = (key, ops.permute_weights(w), w)      # (the filter itself too: its address is the key)
     return hit[1]
 
 

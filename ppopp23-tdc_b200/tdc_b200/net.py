@@ -6,6 +6,7 @@ block size and epilogue) and holds everything the built object points to.  A net
 identity of every tensor it was built from (`fresh` says whether they are still the ones): weights written to or replaced
 mean another build."""
 import ctypes as C
+import threading
 
 import torch
 
@@ -20,6 +21,43 @@ PACKED, PLANES, NCHW = 1, 2, 4
 
 def _key(*tensors):
     return tuple((t._version, t.data_ptr()) if t is not None else None for t in tensors)
+
+
+# ---- work that is done once and read on any stream --------------------------------------------------------------------------
+def _mark(device):
+    """An event behind what the current stream was given so far (None under capture: a replay repeats the work in place)."""
+    if device.index is None or torch.cuda.is_current_stream_capturing():
+        return None
+    event = torch.cuda.Event()
+    event.record()
+    return event
+
+
+class building:
+    """`with building(device):` around work whose results are kept — prepared filters, folded BatchNorms, channel-last copies.  They
+    are shared between nets, and the next net may be built by another thread on another stream: one is built at a time,
+    and its stream first waits for the work of the one before."""
+    _lock, _depth, _last = threading.RLock(), 0, {}
+
+    def __init__(self, device):
+        self.device, self.on = device, _on_device(device)
+
+    def __enter__(self):
+        building._lock.acquire()
+        building._depth += 1
+        self.on.__enter__()
+        last = building._last.get(self.device.index) if building._depth == 1 else None
+        if last is not None and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream().wait_event(last)
+
+    def __exit__(self, *exc):
+        try:
+            if building._depth == 1:
+                building._last[self.device.index] = _mark(self.device) or building._last.get(self.device.index)
+        finally:
+            building._depth -= 1
+            self.on.__exit__(*exc)
+            building._lock.release()
 
 
 class Cache(dict):
@@ -40,6 +78,7 @@ class Net:
         self._h = C.c_void_p()
         self._keep = []                 # everything the launches point to
         self._channels = {-1: Cc}       # tensor -> its channels (-1: the input)
+        self._event, self._streams = None, set()
         self.nchw = False               # which steps the network builders take (programs.py)
         self.clocks = 0.0
         with _on_device(device):
@@ -167,7 +206,21 @@ class Net:
         check(lib.tdc_net_finish(self._h, C.byref(n)))
         self.arena_bytes, self.out_shape = n.value, tuple(out_shape)
         self.arena_floats = max(1, -(-n.value // 4))
+        self._event = _mark(self.device)
         return self
+
+    def meet(self, stream):
+        """Before the first run on a stream: the run waits for what was prepared for the net, wherever that was, and the memory it
+        reads is not given to anyone else while the stream may still be reading it, whatever becomes of the net."""
+        if torch.cuda.is_current_stream_capturing():      # (captures begin on an idle device; what a graph reads is for its owner to keep)
+            return
+        current = torch.cuda.current_stream()
+        if self._event is not None:
+            current.wait_event(self._event)
+        for t in self._keep:
+            if t is not None and t.is_cuda:
+                t.record_stream(current)
+        self._streams.add(stream)
 
     def __call__(self, x, out=None, x_absmax=None, y_absmax=None):
         if out is None:
@@ -175,11 +228,17 @@ class Net:
         arena = x.new_empty(self.arena_floats)
         if x_absmax is None and y_absmax is None and self.device.index == torch.cuda.current_device():
             # (the lean form of the call below: a batch-1 layer is over in less time than the interpreter's detours take)
-            code = lib.tdc_net_run(self._h, x.data_ptr(), None, out.data_ptr(), None, arena.data_ptr(), self.arena_bytes, _stream())
+            stream = _stream()
+            if stream not in self._streams:
+                self.meet(stream)
+            code = lib.tdc_net_run(self._h, x.data_ptr(), None, out.data_ptr(), None, arena.data_ptr(), self.arena_bytes, stream)
             if code:
                 check(code)
             return out
         with _on_device(x.device):
+            stream = _stream()
+            if stream not in self._streams:
+                self.meet(stream)
             check(lib.tdc_net_run(self._h, x.data_ptr(), x_absmax.data_ptr() if x_absmax is not None else None, out.data_ptr(),
-                                  y_absmax.data_ptr() if y_absmax is not None else None, arena.data_ptr(), self.arena_bytes, _stream()))
+                                  y_absmax.data_ptr() if y_absmax is not None else None, arena.data_ptr(), self.arena_bytes, stream))
         return out

@@ -17,7 +17,7 @@ from torch.nn.modules import module as _module
 
 from . import net as N
 from ._lib import ERR_SHAPE, ERR_SMEM, ERR_UNSUPPORTED, NetConv, TdcError, check, lib
-from .ops import _on_device, _stream
+from .ops import _stream
 
 import ctypes as C
 
@@ -52,7 +52,7 @@ def fold_bn(bn):
         n4 = (n + 3) // 4 * 4                                 # scale and shift 16-byte aligned
         buf = torch.empty(2 * n4 + 2, device=dev, dtype=torch.float32)
         scale, shift, bound = buf[:n], buf[n4:n4 + n], buf[2 * n4:]
-        with _on_device(dev):
+        with N.building(dev):
             check(lib.tdc_net_fold_bn(bn.running_var.data_ptr(), bn.running_mean.data_ptr(), bn.weight.data_ptr() if bn.weight is not None else None,
                                       bn.bias.data_ptr() if bn.bias is not None else None, bn.eps, n, scale.data_ptr(), shift.data_ptr(), bound.data_ptr(), _stream()))
         hit = bn.__dict__["_tdc_fold"] = (key, scale, shift, bound)
@@ -514,7 +514,7 @@ def forward(model, x, build):
         elif net or net is False or not cache.plain(model):
             return y if cache.plain(model) else None
         else:
-            with cache.lock, _on_device(x.device):
+            with cache.lock, N.building(x.device):
                 if key not in cache.nets:
                     cache.nets[key] = _build(model, x, build)
                     while len(cache.nets) > Nets.MOST:
@@ -567,7 +567,7 @@ def layer(module, x):
     if net is None:
         while len(cache.nets) >= Nets.MOST:
             cache.nets.pop(next(iter(cache.nets)))
-        with _on_device(x.device):
+        with N.building(x.device):
             net = cache.nets[key] = _build_layer(module, x)
     return net(x) if net else None
 

@@ -16,7 +16,7 @@ import torch
 
 from . import _lib
 from ._lib import TcPlan, TdcError, lib
-from .net import Cache
+from .net import Cache, building
 from .ops import _dev_f32, _epilogue, _on_device, _stream
 
 
@@ -134,14 +134,14 @@ class TcConv:
             return None
         w = self._weight if self._w_layout == _lib.W_KCRS else self._weight.permute(3, 0, 1, 2).contiguous()
         try:
-            with _on_device(x.device):
+            with N.building(x.device):
                 net = N.Net(B, Cc, H, W, x.device)
                 net.conv(net.pack(pack), kind, w, scale, bias, relu, out=N.NCHW, owner=self, name="weight", unbiased=self.unbiased)
+                return net.finish((B, self.K, -(-H // stride), -(-W // stride)))
         except TdcError as e:
             if e.code in (_lib.ERR_SMEM, _lib.ERR_UNSUPPORTED, _lib.ERR_SHAPE):
                 return None
             raise
-        return net.finish((B, self.K, -(-H // stride), -(-W // stride)))
 
     def _packs(self, kind, B, Cc, H, W, stride):
         """Whether the packed form is the faster one, by the estimates of both (dispatch.one_launch_us says where they come
@@ -177,8 +177,11 @@ class TcConv:
                 out = x.new_empty(net.out_shape)
                 xmax = x.__dict__.get("_tdc_absmax")
                 arena = x.new_empty(net.arena_floats)
+                stream = _stream()
+                if stream not in net._streams:
+                    net.meet(stream)
                 code = lib.tdc_net_run(net._h, x.data_ptr(), xmax.data_ptr() if xmax is not None else None, out.data_ptr(), ymax.data_ptr(), arena.data_ptr(),
-                                       net.arena_bytes, _stream())
+                                       net.arena_bytes, stream)
                 if code:
                     _check(code)
                 out._tdc_absmax = ymax
@@ -300,7 +303,8 @@ def cached(owner, name, weight, mode, w_layout=_lib.W_KCRS, general=False):
     key = (weight._version, weight.data_ptr(), tuple(weight.shape))
     hit = store.get((name, mode, w_layout, general))
     if hit is None or hit[0] != key:
-        hit = store[(name, mode, w_layout, general)] = (key, TcConv(weight.detach(), mode, w_layout, general, unbiased=True))
+        with building(weight.device):
+            hit = store[(name, mode, w_layout, general)] = (key, TcConv(weight.detach(), mode, w_layout, general, unbiased=True))
     return hit[1]
 
 

@@ -332,3 +332,46 @@ def test_range_sample_is_spread(N, B, C, H, W):
     net.conv(net.pack(), N.CONV3x3, w, relu=True, out=N.NCHW)
     y = net.finish((B, 8, H, W))(x)
     assert rel(y, F.conv2d(x.double(), w.double(), None, 1, 1).relu()) <= FP32_TOL and tc.status() == 0
+
+
+@pytest.mark.parametrize("what", ["network", "module", "layer"])
+def test_built_on_one_stream_run_on_another(N, what):
+    """What a net was built from is ready before any stream's run reads it, and stays while one reads it: the build waits behind a
+    long kernel, the run is another stream's; then the filters are replaced and their memory is asked for and written while
+    that stream has not come to its run yet."""
+    import tdc_b200 as T
+
+    class HP:
+        ranks = {"l": [32, 32]}
+    torch.manual_seed(5)
+    if what == "network":
+        m, x = T.fill_deterministic(T.tkc_resnet18(precision="auto").eval(), seed=0).cuda(), torch.randn(2, 3, 96, 64, device="cuda")
+        weight = m.layer2[0].conv1.core_kernel
+    elif what == "module":
+        m, x = T.TKConv2dC_B200(64, 64, 3, padding=1, hp_dict=HP, name="l").cuda(), torch.randn(2, 64, 14, 14, device="cuda")
+        m.precision, weight = "fp16x3", m.core_kernel
+    else:
+        m, x = T.TcConv(torch.randn(64, 64, 3, 3, device="cuda"), mode=4), torch.randn(2, 64, 14, 14, device="cuda")
+        m.packed, weight = True, None
+    ref = None
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.no_grad():
+        for repeat in range(2):
+            torch.cuda.synchronize()
+            with torch.cuda.stream(a):
+                torch.cuda._sleep(100_000_000)
+                m(x)
+            with torch.cuda.stream(b):
+                y = m(x)
+                torch.cuda._sleep(100_000_000)
+                late = m(x)
+            if weight is not None:
+                with torch.cuda.stream(a):
+                    weight.mul_(1.0)             # another version: the next call prepares the filters anew
+                    m(x)
+                    junk = [torch.full((n,), float("nan"), device="cuda") for n in (1 << 12, 1 << 14, 1 << 16, 1 << 18, 1 << 20) for _ in range(8)]
+                    del junk
+            torch.cuda.synchronize()
+            ref = m(x) if ref is None else ref
+            torch.cuda.synchronize()
+            assert bool(ref.isfinite().all()) and torch.equal(y, ref) and torch.equal(late, ref)
