@@ -431,8 +431,9 @@ TDC_API void tdc_tkconv_destroy(tdc_tkconv* l);
  * cores read (two fp16 parts per value, fp32-level results as in mode 4), so no step splits or gathers anything again.  A
  * net is built once — tensors are numbered as the steps that make them return — finished, and then run any number of
  * times, on any stream, with an arena of the caller's (16-byte aligned, arena_bytes long; one per run in flight).
- * Building and running make the device that was current at tdc_net_create do the work.  The filters, scales and biases
- * named by the steps are device memory that has to outlive the net.
+ * Building and running make the device that was current at tdc_net_create do the work, whichever is current then (the
+ * stream has to be that device's); tdc_net_filter_prepare and tdc_net_fold_bn have no net and work on the current device.
+ * The filters, scales and biases named by the steps are device memory that has to outlive the net.
  *
  * The reference's counterpart is the forward chain of its end-to-end skeletons
  * (A100-evaluation/EndToEnd/resnet18-tk/src/main.cu:127-155). */

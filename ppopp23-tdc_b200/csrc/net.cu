@@ -138,6 +138,18 @@ struct tdc_net {
 
 namespace {
 
+// Makes a net's device current for as long as it lives: kernels are opened to all of shared memory per device, and a launch on the
+// default stream goes to the current one.
+struct OnDevice {
+    int before = -1;
+    explicit OnDevice(int device) {
+        int now = -1;
+        if (cudaGetDevice(&now) == cudaSuccess && now != device && cudaSetDevice(device) == cudaSuccess) before = now;
+    }
+    ~OnDevice() { if (before >= 0) cudaSetDevice(before); }
+    OnDevice(const OnDevice&) = delete;
+};
+
 unsigned blocks_for(long long items, const Facts& f) {
     long long b = (items + OPS_THREADS - 1) / OPS_THREADS;
     const long long cap = 2ll * f.sms < PACK_SLOTS ? 2ll * f.sms : PACK_SLOTS;     // what is resident: every further block samples the range again
@@ -324,6 +336,7 @@ int tdc_net_add_conv(tdc_net* n, int src, const tdc_net_conv* d, int* out) {
     int mode;
     int rc = describe(n, src, d, &a, &mode);
     if (rc) return rc;
+    const OnDevice here(n->device);
     const Choice c{d->nt, d->mt, d->ks};
     Launch l;
     if (!configure(a, mode, c, n->f, &l, nullptr)) return fail(TDC_ERR_SMEM, "nt=%d mt=%d ks=%d does not fit this convolution", c.nt, c.mt, c.ks);
@@ -579,7 +592,7 @@ int tdc_net_head(tdc_net* n, int src, const float* scale, const float* shift, co
     // few images: a warp per output keeps every SM busy reading the filter; many: tiles reuse both operands
     const bool tile = a.B >= 16;
     const void* fc = a.vec ? (const void*)&fc_tile_kernel<true> : (const void*)&fc_tile_kernel<false>;
-    if (tile) { const int rc = opt_in(fc, n->f.smem_max); if (rc) return rc; }
+    if (tile) { const OnDevice here(n->device); const int rc = opt_in(fc, n->f.smem_max); if (rc) return rc; }
     n->ops.push_back([n, g, a, tile, fc](const RunArgs& r) {
         HeadArgs p = a;
         p.g = reinterpret_cast<float*>(r.arena + n->buffers[g].off); p.y = r.y;
@@ -629,6 +642,7 @@ int tdc_net_run(const tdc_net* n, const float* x, const float* x_absmax, float* 
     if (!n->finished) return fail(TDC_ERR_UNSUPPORTED, "the net is not finished");
     if (arena_bytes < n->arena_bytes) return fail(TDC_ERR_WORKSPACE, "arena of %zu bytes, %zu are needed", arena_bytes, n->arena_bytes);
     if (reinterpret_cast<uintptr_t>(arena) % 16) return fail(TDC_ERR_UNSUPPORTED, "the arena is 16-byte aligned");
+    const OnDevice here(n->device);
     RunArgs r{static_cast<char*>(arena), nullptr, x, x_absmax, y, y_absmax, (cudaStream_t)stream};
     for (const auto& op : n->ops) {
         const cudaError_t e = op(r);
