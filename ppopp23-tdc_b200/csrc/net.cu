@@ -150,6 +150,9 @@ struct OnDevice {
     OnDevice(const OnDevice&) = delete;
 };
 
+// Spaces count positions in 32 bits (Space::Lp, the fast divisions): `pad` zeros per row and image included.
+bool image_fits(long long B, long long H, long long W) { return (H + 2) * (W + 2) < (1ll << 30) && B * (H + 2) * (W + 2) < (1ll << 31); }
+
 unsigned blocks_for(long long items, const Facts& f) {
     long long b = (items + OPS_THREADS - 1) / OPS_THREADS;
     const long long cap = 2ll * f.sms < PACK_SLOTS ? 2ll * f.sms : PACK_SLOTS;     // what is resident: every further block samples the range again
@@ -233,7 +236,7 @@ extern "C" {
 
 int tdc_net_create(tdc_net** out, int B, int C, int H, int W) {
     if (!out) return fail(TDC_ERR_NULL, "out is NULL");
-    if (B <= 0 || C <= 0 || H <= 0 || W <= 0) return fail(TDC_ERR_SHAPE, "B=%d C=%d H=%d W=%d", B, C, H, W);
+    if (B <= 0 || C <= 0 || H <= 0 || W <= 0 || !image_fits(B, H, W)) return fail(TDC_ERR_SHAPE, "B=%d C=%d H=%d W=%d", B, C, H, W);
     Facts f;
     const int rc = facts_of_device(&f);
     if (rc) return rc;
@@ -286,7 +289,7 @@ int tdc_net_conv_plan(tdc_net* n, int src, tdc_net_conv* d) {
 
 int tdc_net_estimate(int B, int C, int H, int W, int split, tdc_net_conv* d) {
     if (!d) return fail(TDC_ERR_NULL, "conv must be non-NULL");
-    if (B <= 0 || C <= 0 || H <= 0 || W <= 0) return fail(TDC_ERR_SHAPE, "B=%d C=%d H=%d W=%d", B, C, H, W);
+    if (B <= 0 || C <= 0 || H <= 0 || W <= 0 || !image_fits(B, H, W)) return fail(TDC_ERR_SHAPE, "B=%d C=%d H=%d W=%d", B, C, H, W);
     Facts f;
     const int rc = facts_of_device(&f);
     if (rc) return rc;
@@ -415,7 +418,7 @@ int tdc_net_add_conv(tdc_net* n, int src, const tdc_net_conv* d, int* out) {
 
 int tdc_net_planes(tdc_net* n, int B, int C, int H, int W, int* out) {
     if (!n || !out) return fail(TDC_ERR_NULL, "net and out must be non-NULL");
-    if (B <= 0 || C <= 0 || H <= 0 || W <= 0) return fail(TDC_ERR_SHAPE, "B=%d C=%d H=%d W=%d", B, C, H, W);
+    if (B <= 0 || C <= 0 || H <= 0 || W <= 0 || !image_fits(B, H, W)) return fail(TDC_ERR_SHAPE, "B=%d C=%d H=%d W=%d", B, C, H, W);
     *out = n->tensor(make_space(B, H, W, 1), C, false, true);
     return TDC_OK;
 }

@@ -61,3 +61,13 @@ def test_the_device_of_a_net(built, tmp_path):
     assert r.returncode == 0, r.stderr
     r = subprocess.run([exe], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.split("\n")[0] == "opened 0 2 launches 0 4 current 0", r.stdout + r.stderr
+
+
+def test_images_whose_positions_do_not_count_in_32_bits_are_refused(built):
+    """50000 x 50000 positions overflow an int, and the sizes computed from it would pass every later check."""
+    import ctypes as C
+    from tdc_b200 import _lib
+    h, d = C.c_void_p(), _lib.NetConv()
+    for B, H, W in ((1, 50000, 50000), (1, 1 << 30, 4), (4096, 1024, 1024)):
+        assert _lib.lib.tdc_net_create(C.byref(h), B, 1, H, W) == _lib.ERR_SHAPE and not h
+        assert _lib.lib.tdc_net_estimate(B, 16, H, W, 0, C.byref(d)) == _lib.ERR_SHAPE
