@@ -523,6 +523,10 @@ TDC_API int tdc_net_head(tdc_net* net, int src, const float* scale, const float*
 TDC_API int tdc_net_finish(tdc_net* net, size_t* arena_bytes);
 /* x_absmax / y_absmax: TDC_TC_ABSMAX_FLOATS partial maxima of |x| known / of |y| wanted (nets that end in NCHW), or NULL. */
 TDC_API int tdc_net_run(const tdc_net* net, const float* x, const float* x_absmax, float* y, float* y_absmax, void* arena, size_t arena_bytes, void* stream);
+/* The same for a net that ends in TDC_NET_NCHW, with scale[K] and bias[K] (or NULL) of the run's own in place of those its last
+ * convolution was built with: one net serves a layer whatever vectors a call brings. */
+TDC_API int tdc_net_run_scaled(const tdc_net* net, const float* x, const float* x_absmax, const float* scale, const float* bias, float* y, float* y_absmax,
+                               void* arena, size_t arena_bytes, void* stream);
 
 #ifdef __cplusplus
 }

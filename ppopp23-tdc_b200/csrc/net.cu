@@ -82,7 +82,10 @@ struct Tensor {
     int slots = 0;                     // partial maxima written so far
 };
 
-struct RunArgs { char* arena; const float* meta; const float* x; const float* x_absmax; float* y; float* y_absmax; cudaStream_t st; };
+struct RunArgs {
+    char* arena; const float* x; const float* x_absmax; float* y; float* y_absmax; cudaStream_t st;
+    bool factors; const float* scale; const float* bias;      // factors: these in place of what the convolution that writes y was built with
+};
 
 }  // namespace
 
@@ -94,7 +97,7 @@ struct tdc_net {
     std::vector<Buffer> buffers;
     std::vector<std::function<cudaError_t(const RunArgs&)>> ops;
     size_t meta_floats = 0, meta_off = 0, arena_bytes = 0;
-    bool finished = false;
+    bool finished = false, packed_y = false;        // packed_y: a convolution on packed activations writes y
 
     int buffer(size_t bytes) {
         Buffer b;
@@ -394,6 +397,7 @@ int tdc_net_add_conv(tdc_net* n, int src, const tdc_net_conv* d, int* out) {
     }
     const int res = d->residual, flags = d->out;
     const bool fresh = d->into < 0;
+    if (id < 0) n->packed_y = true;
     n->ops.push_back([n, src, id, res, flags, into_c, fresh, a, l, fn](const RunArgs& r) {
         Args p = a;
         const Tensor& s = n->tensors[src];
@@ -409,6 +413,7 @@ int tdc_net_add_conv(tdc_net* n, int src, const tdc_net_conv* d, int* out) {
             p.y_slots = m + 1;
         } else {
             p.nchw = r.y; p.y_slots = r.y_absmax; p.y_slots_clear = tdc_tc::ABSMAX_SLOTS;
+            if (r.factors) { p.scale = r.scale; p.bias = r.bias; }      // (the bounds taken from those it was built with serve packed outputs only)
         }
         return launch(fn, dim3(l.grid), l.threads, l.cluster, l.smem, &p, r.st);
     });
@@ -640,19 +645,27 @@ int tdc_net_finish(tdc_net* n, size_t* arena_bytes) {
     return TDC_OK;
 }
 
-int tdc_net_run(const tdc_net* n, const float* x, const float* x_absmax, float* y, float* y_absmax, void* arena, size_t arena_bytes, void* stream) {
-    if (!n || !x || !y || !arena) return fail(TDC_ERR_NULL, "net, x, y and arena must be non-NULL");
+static int run(const tdc_net* n, RunArgs r, size_t arena_bytes) {
+    if (!n || !r.x || !r.y || !r.arena) return fail(TDC_ERR_NULL, "net, x, y and arena must be non-NULL");
     if (!n->finished) return fail(TDC_ERR_UNSUPPORTED, "the net is not finished");
+    if (r.factors && !n->packed_y) return fail(TDC_ERR_UNSUPPORTED, "scale and bias per run go to a net that ends in a convolution on packed activations");
     if (arena_bytes < n->arena_bytes) return fail(TDC_ERR_WORKSPACE, "arena of %zu bytes, %zu are needed", arena_bytes, n->arena_bytes);
-    if (reinterpret_cast<uintptr_t>(arena) % 16) return fail(TDC_ERR_UNSUPPORTED, "the arena is 16-byte aligned");
+    if (reinterpret_cast<uintptr_t>(r.arena) % 16) return fail(TDC_ERR_UNSUPPORTED, "the arena is 16-byte aligned");
     const OnDevice here(n->device);
-    RunArgs r{static_cast<char*>(arena), nullptr, x, x_absmax, y, y_absmax, (cudaStream_t)stream};
     for (const auto& op : n->ops) {
         const cudaError_t e = op(r);
         if (e == cudaErrorUnknown) return TDC_ERR_CUDA;           // a step's entry point has said why
         if (e != cudaSuccess) return fail(TDC_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
     }
     return TDC_OK;
+}
+
+int tdc_net_run(const tdc_net* n, const float* x, const float* x_absmax, float* y, float* y_absmax, void* arena, size_t arena_bytes, void* stream) {
+    return run(n, RunArgs{static_cast<char*>(arena), x, x_absmax, y, y_absmax, (cudaStream_t)stream, false, nullptr, nullptr}, arena_bytes);
+}
+
+int tdc_net_run_scaled(const tdc_net* n, const float* x, const float* x_absmax, const float* scale, const float* bias, float* y, float* y_absmax, void* arena, size_t arena_bytes, void* stream) {
+    return run(n, RunArgs{static_cast<char*>(arena), x, x_absmax, y, y_absmax, (cudaStream_t)stream, true, scale, bias}, arena_bytes);
 }
 
 }  // extern "C"

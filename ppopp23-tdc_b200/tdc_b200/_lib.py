@@ -116,6 +116,7 @@ _PROTOTYPES = {
     "tdc_net_head": (_i, [_p, _i] + [_p] * 4 + [_i]),
     "tdc_net_finish": (_i, [_p, C.POINTER(_sz)]),
     "tdc_net_run": (_i, [_p] * 6 + [_sz, _p]),
+    "tdc_net_run_scaled": (_i, [_p] * 8 + [_sz, _p]),
     "tdc_select_tile": (_i, [_i] * 9 + [C.POINTER(DevInfo), C.POINTER(Tile)]),
     "tdc_tile_info": (_i, [_i] * 9 + [C.POINTER(Tile), C.POINTER(LaunchInfo)]),
     "tdc_tile_cost": (_i, [_i] * 9 + [C.POINTER(Tile), C.POINTER(DevInfo), C.POINTER(C.c_double),

@@ -222,11 +222,12 @@ class Net:
                 t.record_stream(current)
         self._streams.add(stream)
 
-    def __call__(self, x, out=None, x_absmax=None, y_absmax=None):
+    def __call__(self, x, out=None, x_absmax=None, y_absmax=None, factors=None):
+        """`factors`: (scale, bias) of this run, either may be None, in place of those the last convolution was built with."""
         if out is None:
             out = x.new_empty(self.out_shape)
         arena = x.new_empty(self.arena_floats)
-        if x_absmax is None and y_absmax is None and self.device.index == torch.cuda.current_device():
+        if x_absmax is None and y_absmax is None and factors is None and self.device.index == torch.cuda.current_device():
             # (the lean form of the call below: a batch-1 layer is over in less time than the interpreter's detours take)
             stream = _stream()
             if stream not in self._streams:
@@ -239,6 +240,10 @@ class Net:
             stream = _stream()
             if stream not in self._streams:
                 self.meet(stream)
-            check(lib.tdc_net_run(self._h, x.data_ptr(), x_absmax.data_ptr() if x_absmax is not None else None, out.data_ptr(),
-                                  y_absmax.data_ptr() if y_absmax is not None else None, arena.data_ptr(), self.arena_bytes, stream))
+            xm, ym = (t.data_ptr() if t is not None else None for t in (x_absmax, y_absmax))
+            if factors is None:
+                check(lib.tdc_net_run(self._h, x.data_ptr(), xm, out.data_ptr(), ym, arena.data_ptr(), self.arena_bytes, stream))
+            else:
+                s, b = (_dev_f32(t, "scale or bias") if t is not None else None for t in factors)
+                check(lib.tdc_net_run_scaled(self._h, x.data_ptr(), xm, s, b, out.data_ptr(), ym, arena.data_ptr(), self.arena_bytes, stream))
         return out

@@ -52,7 +52,7 @@ class TcConv:
         self.C, self.K, self.R, self.S, self.mode, self.general = Cc, K, R, S, mode, bool(general)
         self._weight, self._w_layout = weight, w_layout
         self._by_nt = {(self.plan.nt, None): (self.plan, self._prepare(self.plan))}   # (output-channel block size, strided-row (stride, padding parity)) -> (plan, prepared filter)
-        self._nets = Cache()                                     # (input shape, stride, padding, epilogue) -> net on packed activations, or None
+        self._nets = Cache()                                     # (input shape, stride, padding, ReLU) -> net on packed activations, or None
         self._plain = Cache()                                    # (input shape, stride, padding) -> what a plain call on it launches
         self._sms = torch.cuda.get_device_properties(weight.device).multi_processor_count
         self._nt_of = {}                                         # (batch, image, flags) -> block size (the rules are library calls)
@@ -110,18 +110,18 @@ class TcConv:
         plan, wt = self._for_image(B, H, W, Ho, Wo, flags)
         return plan, wt, flags | (0x200 if self.unbiased and self.mode != 1 else 0)          # TDC_TC_UNBIASED
 
-    def _net(self, x, scale, bias, relu, stride, padding):
+    def _net(self, x, relu, stride, padding):
         """The net that runs this call on packed activations, or None: another filter than 1x1, 3x3 or 7x7 / 2 in its "same"
-        form, or a shape the one-launch kernel is faster on."""
-        key = (x.shape, stride, padding, relu, scale.data_ptr() if scale is not None else 0, bias.data_ptr() if bias is not None else 0)
+        form, or a shape the one-launch kernel is faster on.  Scale and bias come with each run."""
+        key = (x.shape, stride, padding, relu)
         hit = self._nets.get(key, self)
         if hit is self:
             if len(self._nets) >= 32:
                 self._nets.pop(next(iter(self._nets)))
-            hit = self._nets[key] = self._make_net(x, scale, bias, relu, stride, padding)
+            hit = self._nets[key] = self._make_net(x, relu, stride, padding)
         return hit
 
-    def _make_net(self, x, scale, bias, relu, stride, padding):
+    def _make_net(self, x, relu, stride, padding):
         from . import net as N
         kind, pack = {(1, 1): (N.CONV1x1, N.PACK), (3, 1): (N.CONV3x3, N.PACK), (3, 2): (N.CONV3x3_S2, N.PACK_SPLIT), (1, 2): (N.CONV1x1_S2, N.PACK_SPLIT),
                       (7, 2): (N.CONV7x7_S2, N.PACK_S2D)}.get((self.R, stride), (None, None))
@@ -136,7 +136,7 @@ class TcConv:
         try:
             with N.building(x.device):
                 net = N.Net(B, Cc, H, W, x.device)
-                net.conv(net.pack(pack), kind, w, scale, bias, relu, out=N.NCHW, owner=self, name="weight", unbiased=self.unbiased)
+                net.conv(net.pack(pack), kind, w, None, None, relu, out=N.NCHW, owner=self, name="weight", unbiased=self.unbiased)
                 return net.finish((B, self.K, -(-H // stride), -(-W // stride)))
         except TdcError as e:
             if e.code in (_lib.ERR_SMEM, _lib.ERR_UNSUPPORTED, _lib.ERR_SHAPE):
@@ -218,14 +218,14 @@ class TcConv:
             Ho, Wo = (H - 1) // stride + 1, (W - 1) // stride + 1
         if self.mode == 4 and residual is None and not self.exact_range and self.packed is not False:
             _dev_f32(x, "x")
-            net = self._net(x, scale, bias, relu, stride, padding)
+            net = self._net(x, bool(relu), stride, padding)
             if net is not None:
                 if out is None:
                     out = torch.empty(net.out_shape, device=x.device, dtype=torch.float32)
                 else:
                     _dev_f32(out, "out")
                 ymax = torch.empty(ABSMAX_FLOATS, device=x.device, dtype=torch.float32)
-                net(x, out, getattr(x, "_tdc_absmax", None), ymax)
+                net(x, out, getattr(x, "_tdc_absmax", None), ymax, None if scale is None and bias is None else (scale, bias))
                 out._tdc_absmax = ymax
                 if plain:
                     self._remember(asked, (net, None, None, 0, x.device.index, net.out_shape))

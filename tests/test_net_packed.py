@@ -375,3 +375,24 @@ def test_built_on_one_stream_run_on_another(N, what):
             ref = m(x) if ref is None else ref
             torch.cuda.synchronize()
             assert bool(ref.isfinite().all()) and torch.equal(y, ref) and torch.equal(late, ref)
+
+
+@pytest.mark.parametrize("R,stride", [(1, 1), (3, 2)])
+def test_scale_and_bias_come_with_the_call(N, R, stride):
+    """One net per shape, whatever vectors a call brings: new ones on every call, one of the two, none, and the same memory rewritten."""
+    import tdc_b200 as T
+    x, w, scale, bias = draw(22, 2, 24, 40, 15, 13, R)
+    conv = T.TcConv(w, mode=4, general=stride > 1)
+    conv.packed = True
+    kw = dict(stride=stride, padding=R // 2) if stride > 1 else {}
+    one, zero = torch.ones_like(scale), torch.zeros_like(bias)
+    for k in range(4):
+        s, b = scale * (k + 1), bias - k
+        for sc, bi in ((s, b), (s, None), (None, b), (None, None)):
+            ref = conv64(x, w, stride, one if sc is None else sc, zero if bi is None else bi, True)
+            assert rel(conv(x, sc, bi, None, True, **kw), ref) <= FP32_TOL
+    s = scale.clone()
+    for _ in range(2):
+        assert rel(conv(x, s, bias, None, True, **kw), conv64(x, w, stride, s, bias, True)) <= FP32_TOL
+        s.mul_(-2.0)
+    assert len(conv._nets) == 1
