@@ -301,7 +301,9 @@ x[1, 0, H // 2, W // 2] = 1e5 * float(x.abs().max())
 y = run(x)
 assert bool(y[0].isfinite().all()) and not bool(y[1].isfinite().all()), y
 assert tc.status() == 2
-conv = T.TcConv(torch.randn(K, C, 3, 3, generator=g).cuda(), mode=4)
+x = torch.randn(2, 16, 56, 56, generator=g).cuda()
+x[1, 0, 5, 3] = 1e5 * float(x.abs().max())      # (element 50459: that kernel's sample takes every 49th)
+conv = T.TcConv(torch.randn(K, 16, 3, 3, generator=g).cuda(), mode=4)
 conv.packed = False
 assert not bool(conv(x, relu=True)[1].isfinite().all())
 """
