@@ -37,11 +37,13 @@ class TcConv:
     # one launch that splits and gathers as it goes.  None: where it is the faster of the two (`_packs`)
     packed = None
 
-    def __init__(self, weight, mode=3, w_layout=_lib.W_KCRS, general=False, exact_range=False, unbiased=False):
+    def __init__(self, weight, mode=3, w_layout=_lib.W_KCRS, general=False, exact_range=False, unbiased=False, snapshot=True):
         """weight: [K][C][R][S] (or [C][R][S][K] with w_layout=W_CRSK), fp32 CUDA tensor.  `exact_range` (mode 4): take
         the input's scale from its true maximum (a pass over the input per call) instead of from a sample.  `unbiased`
         (modes 3, 4): put back the expected loss of the tensor core's truncating accumulation (TDC_TC_UNBIASED); sums of
-        small integers are then no longer exact."""
+        small integers are then no longer exact.  `snapshot`: the layer is that of `weight` as it is now; further forms of it (other
+        block sizes, packed) are prepared from a copy when a shape first needs them.  False: from `weight` itself, which the
+        owner then does not write to while the layer is used."""
         self.exact_range, self.unbiased = bool(exact_range), bool(unbiased)
         if w_layout == _lib.W_KCRS:
             K, Cc, R, S = weight.shape
@@ -52,7 +54,9 @@ class TcConv:
         self.C, self.K, self.R, self.S, self.mode, self.general = Cc, K, R, S, mode, bool(general)
         self._weight, self._w_layout = weight, w_layout
         self._by_nt = {(self.plan.nt, None): (self.plan, self._prepare(self.plan))}   # (output-channel block size, strided-row (stride, padding parity)) -> (plan, prepared filter)
-        self._nets = Cache()                                     # (input shape, stride, padding, ReLU) -> net on packed activations, or None
+        if snapshot:
+            self._weight = weight.detach().clone()
+        self._nets = Cache()                                     # (input shape, stride, padding, ReLU, switches) -> net on packed activations, or None
         self._plain = Cache()                                    # (input shape, stride, padding) -> what a plain call on it launches
         self._sms = torch.cuda.get_device_properties(weight.device).multi_processor_count
         self._nt_of = {}                                         # (batch, image, flags) -> block size (the rules are library calls)
@@ -113,7 +117,7 @@ class TcConv:
     def _net(self, x, relu, stride, padding):
         """The net that runs this call on packed activations, or None: another filter than 1x1, 3x3 or 7x7 / 2 in its "same"
         form, or a shape the one-launch kernel is faster on.  Scale and bias come with each run."""
-        key = (x.shape, stride, padding, relu)
+        key = (x.shape, stride, padding, relu, self.unbiased, self.packed)
         hit = self._nets.get(key, self)
         if hit is self:
             if len(self._nets) >= 32:
@@ -170,7 +174,7 @@ class TcConv:
         # and a third of the host time (a small layer is over sooner than the interpreter's way to its launch)
         rec = self._plain.get((x.shape, stride, padding)) if (scale is None and bias is None and residual is None and not relu and out is None) else None
         if rec is not None and rec[4] == x.device.index == torch.cuda.current_device() and x.dtype is torch.float32 and x.is_contiguous() and self.packed is None \
-                and not _TUNING:
+                and self.unbiased is rec[6] and not self.exact_range and not _TUNING:
             net, plan, wt, flags = rec[:4]
             if net is not None:
                 ymax = x.new_empty(ABSMAX_FLOATS)
@@ -228,7 +232,7 @@ class TcConv:
                 net(x, out, getattr(x, "_tdc_absmax", None), ymax, None if scale is None and bias is None else (scale, bias))
                 out._tdc_absmax = ymax
                 if plain:
-                    self._remember(asked, (net, None, None, 0, x.device.index, net.out_shape))
+                    self._remember(asked, (net, None, None, 0, x.device.index, net.out_shape, self.unbiased))
                 return out
         if out is None:
             out = torch.empty((B, self.K, Ho, Wo), device=x.device, dtype=torch.float32)
@@ -240,7 +244,7 @@ class TcConv:
         if self.unbiased and self.mode != 1:
             flags |= 0x200                        # TDC_TC_UNBIASED
         if plain:
-            self._remember(asked, (None, C.byref(plan), wt, flags, x.device.index, (B, self.K, Ho, Wo)))
+            self._remember(asked, (None, C.byref(plan), wt, flags, x.device.index, (B, self.K, Ho, Wo), self.unbiased))
         if self.mode != 4:
             with _on_device(x.device):
                 _check(lib.tdc_conv2d_tc(C.byref(plan), _dev_f32(x, "x"), wt.data_ptr(), _dev_f32(out, "out"),
@@ -304,7 +308,7 @@ def cached(owner, name, weight, mode, w_layout=_lib.W_KCRS, general=False):
     hit = store.get((name, mode, w_layout, general))
     if hit is None or hit[0] != key:
         with building(weight.device):
-            hit = store[(name, mode, w_layout, general)] = (key, TcConv(weight.detach(), mode, w_layout, general, unbiased=True))
+            hit = store[(name, mode, w_layout, general)] = (key, TcConv(weight.detach(), mode, w_layout, general, unbiased=True, snapshot=False))
     return hit[1]
 
 

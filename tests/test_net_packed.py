@@ -398,3 +398,24 @@ def test_scale_and_bias_come_with_the_call(N, R, stride):
         assert rel(conv(x, s, bias, None, True, **kw), conv64(x, w, stride, s, bias, True)) <= FP32_TOL
         s.mul_(-2.0)
     assert len(conv._nets) == 1
+
+
+@pytest.mark.parametrize("C,H,mode", [(64, 14, 4), (256, 7, 4), (64, 56, 4), (64, 14, 3)])
+def test_layer_is_that_of_its_weight_when_it_was_made(N, monkeypatch, C, H, mode):
+    """Forms prepared when a shape first needs them (packed, other block sizes) are those of the weight at construction, and the
+    layer's switches count on every call."""
+    import tdc_b200 as T
+    from tdc_b200 import tc
+    monkeypatch.setattr(tc, "_TUNING", False)
+    x, w, _, _ = draw(23, 2, C, C, H, H, 3)
+    one, zero = torch.ones(C, device="cuda"), torch.zeros(C, device="cuda")
+    conv, ref = T.TcConv(w, mode=mode), conv64(x, w, 1, one, zero, False)
+    fresh = {u: T.TcConv(w.clone(), mode=mode, unbiased=u) for u in (False, True)}
+    w.mul_(3.0)
+    for B in (2, 1, 2):
+        assert rel(conv(x[:B]), ref[:B]) <= FP32_TOL
+    for unbiased in (True, False):
+        conv.unbiased = unbiased
+        assert torch.equal(conv(x), fresh[unbiased](x))
+    conv.exact_range = mode == 4
+    assert rel(conv(x), ref) <= FP32_TOL
