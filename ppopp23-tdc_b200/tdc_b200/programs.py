@@ -104,10 +104,18 @@ def _square(conv, size):
 
 
 def _with_bias(conv, scale, shift):
+    """(conv + bias) * scale + shift, kept on the module: a captured graph reads it after the net it was captured from has made room
+    for another shape's, as it reads the filters and folds kept there."""
     if conv.bias is None:
         return shift
-    b = conv.bias.detach() if scale is None else conv.bias.detach() * scale      # (conv + bias) * scale + shift
-    return b if shift is None else shift + b
+    if scale is None and shift is None:
+        return conv.bias.detach()
+    key = N._key(conv.bias, scale, shift)
+    hit = conv.__dict__.get("_tdc_shift")
+    if hit is None or hit[0] != key:
+        b = conv.bias.detach() if scale is None else conv.bias.detach() * scale
+        hit = conv.__dict__["_tdc_shift"] = (key, b if shift is None else shift + b, conv.bias.detach(), scale, shift)
+    return hit[1]
 
 
 def conv(net, module, x, scale, shift, relu, precision, residual=-1, out=N.PACKED, split=False, into=-1, into_c=0, pool=None):

@@ -253,3 +253,19 @@ def test_filters_and_vectors_match_their_tensor(built):
         with pytest.raises(TdcError) as e:
             call()
         assert e.value.code == 2          # TDC_ERR_SHAPE
+
+
+def test_bias_and_batchnorm_are_folded_once(built):
+    """What a net's launches read lives on the modules: a net that makes room for another shape's takes nothing with it that a graph
+    captured from it still reads."""
+    from tdc_b200 import programs
+    conv, scale, shift = nn.Conv2d(4, 8, 1), torch.rand(8) + 0.5, torch.rand(8)
+    first = programs._with_bias(conv, scale, shift)
+    assert torch.equal(first, shift + conv.bias.detach() * scale) and programs._with_bias(conv, scale, shift) is first
+    with torch.no_grad():
+        conv.bias.add_(1)
+    again = programs._with_bias(conv, scale, shift)
+    assert again is not first and torch.equal(again, shift + conv.bias.detach() * scale)
+    shift.mul_(2)
+    assert torch.equal(programs._with_bias(conv, scale, shift), shift + conv.bias.detach() * scale)
+    assert programs._with_bias(conv, None, None).data_ptr() == conv.bias.data_ptr()
