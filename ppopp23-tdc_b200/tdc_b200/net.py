@@ -60,6 +60,15 @@ class building:
             building._lock.release()
 
 
+def make_room(table, most):
+    """Drops the oldest entries until one more fits (another thread may be at the same table)."""
+    while len(table) >= most:
+        try:
+            table.pop(next(iter(table)), None)
+        except (StopIteration, RuntimeError):
+            pass
+
+
 class Cache(dict):
     """Nets kept on an object that may be copied or pickled: a net is a handle to memory of this process, so a copy starts
     without them."""
@@ -131,7 +140,7 @@ class Net:
 
     def _filter(self, kind, weight, nt, nbytes, scale, bias, owner, name):
         store = owner.__dict__.setdefault("_net_filters", {}) if owner is not None else {}
-        at, key = (name, kind, nt), _key(weight, scale, bias)
+        at, key = (name, kind, nt, scale is None, bias is None), _key(weight, scale, bias)
         hit = store.get(at)
         if hit is None or hit[0] != key:
             w = weight.detach()

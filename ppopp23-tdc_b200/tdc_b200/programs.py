@@ -8,6 +8,7 @@ where something changed (a weight written to or replaced, a submodule exchanged,
 the forward runs again.  A network that a net cannot express (an exotic stride, a hook that wants to see a layer) runs
 layer by layer.  So does one with a module of another kind in a place that the layer-by-layer forward CALLS (stages, blocks, the
 average pool, the classifier): a net stands for the forwards of the exact classes named in the builders, no subclass's."""
+import functools
 import math
 import threading
 
@@ -68,23 +69,34 @@ class At:
         self.id, self.C, self.H, self.W, self.split = id, Cc, H, W, split
 
 
-def _estimate(B, Cc, H, W, split, kind, K, residual, out, pool=0):
+def _estimate(*layer):
+    return _estimate_on(torch.cuda.current_device(), *layer)
+
+
+def _pooled_estimates(*layer):
+    return _pooled_estimates_on(torch.cuda.current_device(), *layer)
+
+
+# (remembered: a module weighs several forms that share steps, a network repeats its blocks)
+@functools.lru_cache(maxsize=8192)
+def _estimate_on(device, B, Cc, H, W, split, kind, K, residual, out, pool=0):
     if pool:
-        return min(_pooled_estimates(B, Cc, H, W, split, kind, K, out, pool))
+        return min(_pooled_estimates_on(device, B, Cc, H, W, split, kind, K, out, pool))
     d = NetConv()
     d.kind, d.K, d.residual, d.out, d.into = kind, K, 0 if residual else -1, out, -1
     check(lib.tdc_net_estimate(B, Cc, H, W, int(split), C.byref(d)))
     return d.clocks
 
 
-def _pooled_estimates(B, Cc, H, W, split, kind, K, out, pool):
+@functools.lru_cache(maxsize=8192)
+def _pooled_estimates_on(device, B, Cc, H, W, split, kind, K, out, pool):
     """Clocks of a convolution whose epilogue pools (infinite where no kernel does), and of the two steps one by one: pooling
     reads fp32 planes and leaves `out`, from HBM where it moves more than L2 holds (bytes per clock of the whole chip)."""
     d = NetConv()
     d.kind, d.K, d.residual, d.out, d.into, d.relu, d.pool = kind, K, -1, out, -1, 1, pool
     one = d.clocks if lib.tdc_net_estimate(B, Cc, H, W, int(split), C.byref(d)) == 0 else math.inf
     size = 4.0 * B * K * H * W * (1 + 0.25 * bin(out).count("1"))
-    return one, _estimate(B, Cc, H, W, split, kind, K, False, N.PLANES) + 4000.0 + size / (2600.0 if size > 80e6 else 6500.0)
+    return one, _estimate_on(device, B, Cc, H, W, split, kind, K, False, N.PLANES) + 4000.0 + size / (2600.0 if size > 80e6 else 6500.0)
 
 
 def _pool_of(m):
@@ -455,7 +467,7 @@ class Nets:
     keys of every table of children, parameters and buffers, and the plain attributes the builders read."""
     READ = ("stride", "padding", "dilation", "groups", "kernel_size", "ceil_mode", "output_size", "eps", "in_channels", "out_channels", "in_rank", "out_rank", "rank",
             "num_features", "num_input_features", "num_output_features", "growth_rate", "in_features", "out_features", "downsample")
-    MOST = 16                     # shapes kept: the oldest goes first
+    MOST = 256                    # shapes kept, the oldest goes first: a net is 30 - 200 KB of host memory (filters live on the modules)
 
     def __init__(self, model=None):
         self.nets, self.lock = {}, threading.Lock()
@@ -524,9 +536,8 @@ def forward(model, x, build):
         else:
             with cache.lock, N.building(x.device):
                 if key not in cache.nets:
+                    N.make_room(cache.nets, Nets.MOST)
                     cache.nets[key] = _build(model, x, build)
-                    while len(cache.nets) > Nets.MOST:
-                        cache.nets.pop(next(iter(cache.nets)))
     return None
 
 
@@ -548,6 +559,7 @@ def _build(model, x, build):
 # ---- one Tucker module -------------------------------------------------------------------------------------------------
 class _LayerNet:
     """A module's nets by input shape, precision and device, and the factors they were built from."""
+    MOST = 1024                   # (a few KB each)
 
     def __init__(self):
         self.nets, self.mark = {}, None
@@ -573,8 +585,7 @@ def layer(module, x):
     key = (x.shape, module.precision, x.device.index, module.stride, module.padding, module.dilation, module.groups)
     net = cache.nets.get(key)
     if net is None:
-        while len(cache.nets) >= Nets.MOST:
-            cache.nets.pop(next(iter(cache.nets)))
+        N.make_room(cache.nets, _LayerNet.MOST)
         with N.building(x.device):
             net = cache.nets[key] = _build_layer(module, x)
     return net(x) if net else None

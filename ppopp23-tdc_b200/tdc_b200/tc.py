@@ -16,7 +16,7 @@ import torch
 
 from . import _lib
 from ._lib import TcPlan, TdcError, lib
-from .net import Cache, building
+from .net import Cache, building, make_room
 from .ops import _dev_f32, _epilogue, _on_device, _stream
 
 
@@ -98,9 +98,10 @@ class TcConv:
             hit = self._by_nt[(nt, rows)] = (plan, self._prepare(plan))
         return hit
 
+    MOST = 1024          # shapes kept, the oldest goes first
+
     def _remember(self, asked, rec):
-        if len(self._plain) >= 64:
-            self._plain.clear()
+        make_room(self._plain, self.MOST)
         self._plain[asked] = rec
 
     def step(self, B, H, W, stride, padding):
@@ -120,8 +121,7 @@ class TcConv:
         key = (x.shape, stride, padding, relu, self.unbiased, self.packed)
         hit = self._nets.get(key, self)
         if hit is self:
-            if len(self._nets) >= 32:
-                self._nets.pop(next(iter(self._nets)))
+            make_room(self._nets, self.MOST)
             hit = self._nets[key] = self._make_net(x, relu, stride, padding)
         return hit
 

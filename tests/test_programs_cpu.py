@@ -269,3 +269,30 @@ def test_bias_and_batchnorm_are_folded_once(built):
     shift.mul_(2)
     assert torch.equal(programs._with_bias(conv, scale, shift), shift + conv.bias.detach() * scale)
     assert programs._with_bias(conv, None, None).data_ptr() == conv.bias.data_ptr()
+
+
+def test_rotating_shapes_stay_built(P):
+    """Forty input sizes in turn: each is built once.  The table is bounded all the same, and threads may make room at once."""
+    import threading
+    from tdc_b200 import net as N
+    model, call = make(P, "vgg")
+    for _ in range(2):
+        for i in range(40):
+            assert call(H=16 + i) is not None
+    assert len(Steps.made) == 40
+    for i in range(P.Nets.MOST):
+        call(H=100 + i)
+    assert len(model._nets.nets) == P.Nets.MOST
+    table, wrong = {i: i for i in range(500)}, []
+
+    def work(k):
+        try:
+            for i in range(2000):
+                N.make_room(table, 400)
+                table[(k, i)] = 1
+        except Exception as e:      # noqa: BLE001
+            wrong.append(e)
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong and len(table) <= 408
