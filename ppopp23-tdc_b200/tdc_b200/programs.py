@@ -574,7 +574,9 @@ class _LayerNet:
 def layer(module, x):
     """A Tucker module's output for a contiguous fp32 x through its net, or None where it has to run step by step."""
     p = module._parameters
-    first, core, last, bias = p["first_kernel"], p["core_kernel"], p["last_kernel"], p["bias"]
+    first, core, last, bias = p.get("first_kernel"), p.get("core_kernel"), p.get("last_kernel"), p.get("bias")
+    if first is None or core is None or last is None:      # parametrised or pruned: they are made anew on every access
+        return None
     mark = (first._version, first.data_ptr(), core._version, core.data_ptr(), last._version, last.data_ptr(),
             None if bias is None else (bias._version, bias.data_ptr()))
     cache = module.__dict__.get("_layer_net")

@@ -296,3 +296,15 @@ def test_rotating_shapes_stay_built(P):
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not wrong and len(table) <= 408
+
+
+def test_parametrised_factors_run_step_by_step(built):
+    """A parametrised or pruned factor is no parameter of the module any more, and is made anew on every access."""
+    import tdc_b200 as T
+    from tdc_b200 import programs
+
+    class HP:
+        ranks = {"l": [8, 8]}
+    m = T.TKConv2dC_B200(16, 16, 3, padding=1, hp_dict=HP, name="l")
+    nn.utils.parametrize.register_parametrization(m, "first_kernel", nn.Identity())
+    assert programs.layer(m, torch.zeros(1, 16, 8, 8)) is None
