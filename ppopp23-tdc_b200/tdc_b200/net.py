@@ -88,6 +88,7 @@ class Net:
         self._keep = []                 # everything the launches point to
         self._channels = {-1: Cc}       # tensor -> its channels (-1: the input)
         self._event, self._streams = None, set()
+        self.leaves_range = False       # a run writes the partial maxima of |y| it is given room for
         self.nchw = False               # which steps the network builders take (programs.py)
         self.clocks = 0.0
         with _on_device(device):
@@ -131,6 +132,7 @@ class Net:
             d.nt, d.mt, d.ks = tile
         check(lib.tdc_net_conv_plan(self._h, src, C.byref(d)))
         self.clocks += d.clocks
+        self.leaves_range |= out == NCHW
         flt = self._filter(kind, weight, d.nt, d.filter_bytes, scale, bias, owner, name)
         d.filter = flt.data_ptr()
         self._keep += [flt, scale, bias]
@@ -174,6 +176,7 @@ class Net:
         d = NetNchw()
         d.K, d.R, d.S, d.stride, d.pad, d.flags, d.residual, d.relu = K, R, R, stride, pad, flags, residual, int(relu)
         d.to_y = int(to_y)
+        self.leaves_range |= bool(to_y) and plan is not None and plan.mode == 4
         d.plan = C.pointer(plan) if plan is not None else None
         d.filter = flt.data_ptr()
         d.scale = _dev_f32(scale, "scale") if scale is not None else None
@@ -236,12 +239,13 @@ class Net:
         if out is None:
             out = x.new_empty(self.out_shape)
         arena = x.new_empty(self.arena_floats)
-        if x_absmax is None and y_absmax is None and factors is None and self.device.index == torch.cuda.current_device():
+        if factors is None and self.device.index == torch.cuda.current_device():
             # (the lean form of the call below: a batch-1 layer is over in less time than the interpreter's detours take)
             stream = _stream()
             if stream not in self._streams:
                 self.meet(stream)
-            code = lib.tdc_net_run(self._h, x.data_ptr(), None, out.data_ptr(), None, arena.data_ptr(), self.arena_bytes, stream)
+            code = lib.tdc_net_run(self._h, x.data_ptr(), None if x_absmax is None else x_absmax.data_ptr(), out.data_ptr(),
+                                   None if y_absmax is None else y_absmax.data_ptr(), arena.data_ptr(), self.arena_bytes, stream)
             if code:
                 check(code)
             return out

@@ -169,6 +169,24 @@ def _epilogue(scale, bias, residual, relu):
     return e
 
 
+ABSMAX_FLOATS = 1024      # TDC_TC_ABSMAX_FLOATS
+
+
+def leave_range(y, absmax):
+    """Keeps on y the partial maxima of |y| that its kernel wrote, for the convolution that reads y next."""
+    y._tdc_absmax, y._tdc_absmax_at = absmax, None if y.is_inference() else y._version
+
+
+def range_of(x):
+    """The partial maxima kept on x, or None: there are none, or x was written to since."""
+    d = x.__dict__
+    hit = d.get("_tdc_absmax")
+    if hit is None:
+        return None
+    at = d.get("_tdc_absmax_at")
+    return hit if at is None or at == x._version else None
+
+
 POOL_MAX, POOL_AVG_INCLUDE_PAD, POOL_AVG_EXCLUDE_PAD = 0, 1, 2
 
 
@@ -187,9 +205,9 @@ def pool2d(x, kernel_size, stride=None, padding=0, mode=POOL_MAX, out=None):
         code = lib.tdc_pool2d_f32(_dev_f32(x, "x"), _dev_f32(out, "out"), B, Cc, H, W, kh, kw, padding, stride, mode, _stream())
     if code != _lib.OK:
         raise TdcError(code, "tdc_pool2d_f32: window %dx%d stride %d padding %d on %dx%d" % (kh, kw, stride, padding, H, W))
-    bound = getattr(x, "_tdc_absmax", None)
+    bound = range_of(x)
     if bound is not None:      # no pooling mode raises the largest magnitude: the input's bound holds for the output
-        out._tdc_absmax = bound
+        leave_range(out, bound)
     return out
 
 

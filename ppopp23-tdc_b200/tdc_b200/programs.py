@@ -18,7 +18,7 @@ from torch.nn.modules import module as _module
 
 from . import net as N
 from ._lib import ERR_SHAPE, ERR_SMEM, ERR_UNSUPPORTED, NetConv, TdcError, check, lib
-from .ops import _stream
+from .ops import ABSMAX_FLOATS, _stream, leave_range, range_of
 
 import ctypes as C
 
@@ -590,7 +590,15 @@ def layer(module, x):
         N.make_room(cache.nets, _LayerNet.MOST)
         with N.building(x.device):
             net = cache.nets[key] = _build_layer(module, x)
-    return net(x) if net else None
+    if not net:
+        return None
+    if not net.leaves_range:
+        return net(x, None, range_of(x))
+    # (from module to module, and from and to TcConv, the exact range: only the first of a chain samples)
+    ymax = x.new_empty(ABSMAX_FLOATS)
+    y = net(x, None, range_of(x), ymax)
+    leave_range(y, ymax)
+    return y
 
 
 def _one_launch_wins(module, x):

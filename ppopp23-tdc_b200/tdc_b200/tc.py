@@ -17,10 +17,7 @@ import torch
 from . import _lib
 from ._lib import TcPlan, TdcError, lib
 from .net import Cache, building, make_room
-from .ops import _dev_f32, _epilogue, _on_device, _stream
-
-
-ABSMAX_FLOATS = 1024      # TDC_TC_ABSMAX_FLOATS
+from .ops import ABSMAX_FLOATS, _dev_f32, _epilogue, _on_device, _stream, leave_range, range_of
 
 
 def _check(code):
@@ -179,7 +176,7 @@ class TcConv:
             if net is not None:
                 ymax = x.new_empty(ABSMAX_FLOATS)
                 out = x.new_empty(net.out_shape)
-                xmax = x.__dict__.get("_tdc_absmax")
+                xmax = range_of(x)
                 arena = x.new_empty(net.arena_floats)
                 stream = _stream()
                 if stream not in net._streams:
@@ -188,7 +185,7 @@ class TcConv:
                                        net.arena_bytes, stream)
                 if code:
                     _check(code)
-                out._tdc_absmax = ymax
+                leave_range(out, ymax)
                 return out
             B, _, H, W = x.shape
             out = x.new_empty(rec[5])
@@ -196,10 +193,10 @@ class TcConv:
                 code = lib.tdc_conv2d_tc(plan, x.data_ptr(), wt.data_ptr(), out.data_ptr(), B, H, W, None, flags, _stream())
             else:
                 ymax = x.new_empty(ABSMAX_FLOATS)
-                xmax = x.__dict__.get("_tdc_absmax")
+                xmax = range_of(x)
                 code = lib.tdc_conv2d_tc_ranged(plan, x.data_ptr(), wt.data_ptr(), out.data_ptr(), B, H, W, None, flags,
                                                 xmax.data_ptr() if xmax is not None else None, ymax.data_ptr(), _stream())
-                out._tdc_absmax = ymax
+                leave_range(out, ymax)
             if code:
                 _check(code)
             return out
@@ -229,8 +226,8 @@ class TcConv:
                 else:
                     _dev_f32(out, "out")
                 ymax = torch.empty(ABSMAX_FLOATS, device=x.device, dtype=torch.float32)
-                net(x, out, getattr(x, "_tdc_absmax", None), ymax, None if scale is None and bias is None else (scale, bias))
-                out._tdc_absmax = ymax
+                net(x, out, range_of(x), ymax, None if scale is None and bias is None else (scale, bias))
+                leave_range(out, ymax)
                 if plain:
                     self._remember(asked, (net, None, None, 0, x.device.index, net.out_shape, self.unbiased))
                 return out
@@ -250,7 +247,7 @@ class TcConv:
                 _check(lib.tdc_conv2d_tc(C.byref(plan), _dev_f32(x, "x"), wt.data_ptr(), _dev_f32(out, "out"),
                                          B, H, W, C.byref(e), flags, _stream()))
             return out
-        xmax = getattr(x, "_tdc_absmax", None)
+        xmax = range_of(x)
         if xmax is None and self.exact_range:
             flags |= 0x100                        # TDC_TC_EXACT_RANGE
         ymax = torch.empty(ABSMAX_FLOATS, device=x.device, dtype=torch.float32)
@@ -258,7 +255,7 @@ class TcConv:
             _check(lib.tdc_conv2d_tc_ranged(C.byref(plan), _dev_f32(x, "x"), wt.data_ptr(), _dev_f32(out, "out"),
                                             B, H, W, C.byref(e), flags, xmax.data_ptr() if xmax is not None else None,
                                             ymax.data_ptr(), _stream()))
-        out._tdc_absmax = ymax
+        leave_range(out, ymax)
         return out
 
 

@@ -419,3 +419,32 @@ def test_layer_is_that_of_its_weight_when_it_was_made(N, monkeypatch, C, H, mode
         assert torch.equal(conv(x), fresh[unbiased](x))
     conv.exact_range = mode == 4
     assert rel(conv(x), ref) <= FP32_TOL
+
+
+def test_modules_pass_their_range_on(N):
+    """The exact range goes from layer to module to module: a value far beyond what a sample would see stays in the headroom of none.
+    A tensor that was written to since is sampled."""
+    import tdc_b200 as T
+    from tdc_b200 import tc
+
+    class HP:
+        ranks = {"l": [16, 16]}
+    torch.manual_seed(6)
+    C, H = 32, 40
+    first = T.TcConv(torch.randn(C, C, 1, 1, device="cuda"), mode=4, exact_range=True)
+    for precision in ("auto", "fp16x3"):
+        m = T.TKConv2dC_B200(C, C, 3, padding=1, bias=False, hp_dict=HP, name="l").cuda()
+        m.precision = precision
+        x = torch.randn(2, C, H, H, device="cuda")
+        x[1, 3, 7, 9] = 1e5 * float(x.abs().max())
+
+        def tucker(x):
+            return F.conv2d(F.conv2d(F.conv2d(x.double(), m.first_kernel.double()), m.core_kernel.double(), None, 1, 1), m.last_kernel.double())
+        with torch.no_grad():
+            y = first(x)
+            z = m(m(y))
+            assert rel(z, tucker(tucker(y))) <= FP32_TOL and tc.status() == 0
+            assert float(z._tdc_absmax.max()) == float(z.abs().max())
+            y = m(torch.randn(2, C, H, H, device="cuda"))
+            y.mul_(1e6)                                 # what it carries is no bound any more
+            assert rel(m(y), tucker(y)) <= FP32_TOL and tc.status() == 0

@@ -308,3 +308,17 @@ def test_parametrised_factors_run_step_by_step(built):
     m = T.TKConv2dC_B200(16, 16, 3, padding=1, hp_dict=HP, name="l")
     nn.utils.parametrize.register_parametrization(m, "first_kernel", nn.Identity())
     assert programs.layer(m, torch.zeros(1, 16, 8, 8)) is None
+
+
+def test_range_of_a_tensor_ends_when_it_is_written_to():
+    from tdc_b200 import ops
+    y, bound = torch.zeros(4), torch.ones(8)
+    assert ops.range_of(y) is None
+    ops.leave_range(y, bound)
+    assert ops.range_of(y) is bound
+    y.view(2, 2).add_(1)
+    assert ops.range_of(y) is None
+    with torch.inference_mode():          # (no version to compare)
+        z = torch.zeros(4)
+        ops.leave_range(z, bound)
+        assert ops.range_of(z) is bound
