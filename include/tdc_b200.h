@@ -518,7 +518,8 @@ TDC_API int tdc_net_nchw_pool(tdc_net* net, int src, int k, int stride, int pad,
 TDC_API int tdc_net_nchw_buffer(tdc_net* net, int C, int H, int W, int* out_tensor);
 TDC_API int tdc_net_nchw_affine(tdc_net* net, int src, int channels, const float* scale, const float* shift, int relu,
                                 int into, int into_c, int* out_tensor);
-/* Global average (after an optional BatchNorm + ReLU) and classifier: y [B][N].  The source has fp32 planes or is NCHW. */
+/* Global average (after an optional BatchNorm + ReLU) and classifier: y [B][N]; w NULL: the averages alone, y [B][C].  The source
+ * has fp32 planes or is NCHW. */
 TDC_API int tdc_net_head(tdc_net* net, int src, const float* scale, const float* shift, const float* w, const float* bias, int N);
 TDC_API int tdc_net_finish(tdc_net* net, size_t* arena_bytes);
 /* x_absmax / y_absmax: TDC_TC_ABSMAX_FLOATS partial maxima of |x| known / of |y| wanted (nets that end in NCHW), or NULL. */

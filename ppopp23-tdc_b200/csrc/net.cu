@@ -575,9 +575,9 @@ int tdc_net_nchw_affine(tdc_net* n, int src, int channels, const float* scale, c
 }
 
 int tdc_net_head(tdc_net* n, int src, const float* scale, const float* shift, const float* w, const float* bias, int N) {
-    if (!n || !w) return fail(TDC_ERR_NULL, "net and w must be non-NULL");
+    if (!n) return fail(TDC_ERR_NULL, "net must be non-NULL");
     if (!n->has(src) || (n->tensors[src].nchw < 0 && (n->tensors[src].f4 < 0 || n->tensors[src].s.split_B))) return fail(TDC_ERR_UNSUPPORTED, "the head reads fp32 planes or an NCHW tensor");
-    if (N <= 0) return fail(TDC_ERR_SHAPE, "N=%d", N);
+    if (w && N <= 0) return fail(TDC_ERR_SHAPE, "N=%d", N);
     const Tensor x = n->tensors[src];
     HeadArgs a{};
     a.B = n->B; a.C = x.C; a.N = N;
@@ -587,15 +587,16 @@ int tdc_net_head(tdc_net* n, int src, const float* scale, const float* shift, co
     a.scale = scale; a.shift = shift; a.w = w; a.bias = bias;
     a.vec = a.C % 4 == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0;
     n->use(planes ? x.f4 : x.nchw);
-    const int g = n->buffer(sizeof(float) * (size_t)a.B * a.C);
+    const int g = w ? n->buffer(sizeof(float) * (size_t)a.B * a.C) : -1;
     const long long warps = (long long)a.B * (planes ? (a.C + 15) / 16 : a.C);
     const unsigned gap_grid = (unsigned)std::min<long long>((warps + 7) / 8, (long long)n->f.sms * 8);
     n->ops.push_back([n, src, g, a, planes, gap_grid](const RunArgs& r) {
         HeadArgs p = a;
         p.x = planes ? n->f4_at(r, n->tensors[src]) : n->nchw_at(r, src);
-        p.g = reinterpret_cast<float*>(r.arena + n->buffers[g].off);
+        p.g = g < 0 ? r.y : reinterpret_cast<float*>(r.arena + n->buffers[g].off);
         return launch(planes ? (const void*)&gap_kernel : (const void*)&gap_nchw_kernel, dim3(gap_grid), HEAD_THREADS, 1, 0, &p, r.st);
     });
+    if (!w) return TDC_OK;
     n->use(g);
     // few images: a warp per output keeps every SM busy reading the filter; many: tiles reuse both operands
     const bool tile = a.B >= 16;

@@ -228,7 +228,7 @@ class TKDenseNet(nn.Module):
 
     def forward(self, x):
         if x.is_cuda and not self.training:
-            y = programs.forward(self, x.contiguous().float(), programs.build_densenet)
+            y = programs.forward(self, x.contiguous().float(), programs.build_densenet, self.classifier)
             if y is not None:
                 return y
         x = self.forward_features(x)

@@ -89,7 +89,7 @@ class Net:
         self._channels = {-1: Cc}       # tensor -> its channels (-1: the input)
         self._event, self._streams = None, set()
         self.leaves_range = False       # a run writes the partial maxima of |y| it is given room for
-        self.nchw = False               # which steps the network builders take (programs.py)
+        self.nchw, self.features = False, False      # which steps the network builders take, and whether they end at the classifier (programs.py)
         self.clocks = 0.0
         with _on_device(device):
             check(lib.tdc_net_create(C.byref(self._h), B, Cc, H, W))
@@ -205,13 +205,18 @@ class Net:
                                       int(relu), into, into_c, C.byref(t)))
         return t.value if into >= 0 else self._made(t.value, channels_out)
 
-    def head(self, src, weight, bias, scale=None, shift=None):
-        weight, bias = weight.detach(), bias.detach() if bias is not None else None      # (aliases: the launches read this memory)
-        self._per_channel(self._channels.get(src, -1), weight[0], scale, shift)
-        self._per_channel(weight.shape[0], bias)
+    def head(self, src, weight=None, bias=None, scale=None, shift=None):
+        """Global average and classifier; without a weight the averages alone."""
+        self._per_channel(self._channels.get(src, -1), scale, shift)
+        w = b = None
+        if weight is not None:
+            weight, bias = weight.detach(), bias.detach() if bias is not None else None      # (aliases: the launches read this memory)
+            self._per_channel(self._channels.get(src, -1), weight[0])
+            self._per_channel(weight.shape[0], bias)
+            w, b = _dev_f32(weight, "weight"), _dev_f32(bias, "bias") if bias is not None else None
         self._keep += [weight, bias, scale, shift]
         check(lib.tdc_net_head(self._h, src, scale.data_ptr() if scale is not None else None, shift.data_ptr() if shift is not None else None,
-                               _dev_f32(weight, "weight"), bias.data_ptr() if bias is not None else None, weight.shape[0]))
+                               w, b, weight.shape[0] if weight is not None else 0))
 
     def finish(self, out_shape):
         n = C.c_size_t()

@@ -14,6 +14,7 @@ import threading
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 from torch.nn.modules import module as _module
 
 from . import net as N
@@ -267,11 +268,35 @@ def pool_max(net, m, x, out):
     return lambda **kw: At(net.pool(x.id, k, s, p, out=out, **kw), x.C, H, W)
 
 
+# ---- the classifier ----------------------------------------------------------------------------------------------------
+def native_classifier(head, x):
+    """What identifies a classifier that a net's last launch stands for, or None where `head` has to be called on the averages:
+    another module than a Linear on fp32 memory, hooks, and whatever torch does around a call — gradients, autocast, forward-mode
+    derivatives, function transforms, dispatch modes."""
+    if type(head) is not nn.Linear or "forward" in head.__dict__ or head._forward_hooks or head._forward_pre_hooks or head._backward_hooks or head._backward_pre_hooks:
+        return None
+    w, b = head._parameters.get("weight"), head._parameters.get("bias")
+    if w is None or (torch.is_grad_enabled() and (w.requires_grad or (b is not None and b.requires_grad))) or torch.is_autocast_enabled(x.device.type) \
+            or forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack():
+        return None
+    if any(t is not None and (t.dtype != torch.float32 or t.device != x.device or not t.is_contiguous()) for t in (w, b)):
+        return None
+    return (w.data_ptr(), None if b is None else b.data_ptr(), w.shape)
+
+
+def classify(net, x, head, scale=None, shift=None):
+    """The end of a network: averages and classifier, or (net.features) the averages that `head` is called on."""
+    if net.features:
+        net.head(x.id, None, None, scale, shift)
+        return net.finish((net.shape[0], x.C))
+    net.head(x.id, head.weight, head.bias, scale, shift)
+    return net.finish((net.shape[0], head.weight.shape[0]))
+
+
 # ---- the networks ----------------------------------------------------------------------------------------------------
 def build_resnet(model, net, precision):
     from .resnet import TKBasicBlock, TKBottleneck
     _average_to_one(model.avgpool)
-    _exact(model.fc, nn.Linear)
     s, b, _ = fold_bn(model.bn1)
     blocks = [_exact(m, TKBasicBlock, TKBottleneck) for layer in (model.layer1, model.layer2, model.layer3, model.layer4) for m in _exact(layer, nn.Sequential)]
     wide = [type(m) is TKBottleneck for m in blocks]
@@ -304,8 +329,7 @@ def build_resnet(model, net, precision):
         if strided(i + 1) and o & N.PLANES:
             raise NotExpressible
         x = conv(net, last, out, s2, b2, True, precision, residual=identity.id, out=o, split=strided(i + 1))
-    net.head(x.id, model.fc.weight, model.fc.bias)
-    return net.finish((net.shape[0], model.fc.out_features))
+    return classify(net, x, model.fc)
 
 
 def build_vgg(model, net, precision):
@@ -313,7 +337,6 @@ def build_vgg(model, net, precision):
     from .vgg import TKVGG
     if type(model).forward_features is not TKVGG.forward_features:
         raise NotExpressible
-    _exact(model.head.fc, nn.Linear)
     mods = list(model.features)
     x, i = None, 0
     B, Cc, H, W = net.shape
@@ -353,8 +376,7 @@ def build_vgg(model, net, precision):
         x = conv(net, m, x, scale, shift, relu, precision, out=out, pool=pool)
     if x is None:
         raise NotExpressible
-    net.head(x.id, model.head.fc.weight, model.head.fc.bias)
-    return net.finish((B, model.head.fc.out_features))
+    return classify(net, x, model.head.fc)
 
 
 def build_densenet(model, net, precision):
@@ -362,7 +384,6 @@ def build_densenet(model, net, precision):
     if type(model).forward_features is not TKDenseNet.forward_features:
         raise NotExpressible
     _average_to_one(model.global_pool)
-    _exact(model.classifier, nn.Linear)
     for name, m in model.features.named_children():
         if name.startswith(("denseblock", "transition")) and type(_exact(m, TKDenseBlock, TKDenseTransition)) is TKDenseBlock:
             for layer in m.values():
@@ -409,8 +430,7 @@ def build_densenet(model, net, precision):
     if buf is None:
         raise NotExpressible
     s, b, _ = fold_bn(f.norm5)
-    net.head(buf, model.classifier.weight, model.classifier.bias, s, b)
-    return net.finish((B, model.classifier.out_features))
+    return classify(net, At(buf, f.norm5.num_features, H, W), model.classifier, s, b)
 
 
 def build_densenet_nchw(model, net, precision):
@@ -452,8 +472,7 @@ def build_densenet_nchw(model, net, precision):
         elif name.startswith(("denseblock", "transition")):
             raise NotExpressible
     s, b, _ = fold_bn(f.norm5)
-    net.head(x.id, model.classifier.weight, model.classifier.bias, s, b)
-    return net.finish((net.shape[0], model.classifier.out_features))
+    return classify(net, x, model.classifier, s, b)
 
 
 def _pooled(m, n):
@@ -469,12 +488,14 @@ class Nets:
             "num_features", "num_input_features", "num_output_features", "growth_rate", "in_features", "out_features", "downsample")
     MOST = 256                    # shapes kept, the oldest goes first: a net is 30 - 200 KB of host memory (filters live on the modules)
 
-    def __init__(self, model=None):
+    def __init__(self, model=None, head=None):
         self.nets, self.lock = {}, threading.Lock()
+        self.classifier = None                                # of the nets that run it themselves
         self.parts, self.tensors, self.modules, self.mark = [], [], [], None
         self.orders, self.sizes, self.lengths, self.read, self.values = [], [], [], [], []
         if model is not None:
-            self.modules = list(model.modules())[1:]          # (not the model itself: it holds this object)
+            apart = set(head.modules())                       # called, or compared by its tensors' addresses (native_classifier)
+            self.modules = [m for m in model.modules() if m not in apart and m is not model]      # (not the model itself: it holds this object)
             for m in [model] + self.modules:
                 self.parts += [(m._modules, k, c) for k, c in m._modules.items()]
                 for d in (m._parameters, m._buffers):
@@ -520,33 +541,38 @@ class Nets:
             return False
 
 
-def forward(model, x, build):
-    """The model's output for x through its net, or None where it has to run layer by layer."""
+def forward(model, x, build, head):
+    """The model's output for x through its net, or None where it has to run layer by layer.  `head`: its classifier."""
+    native = native_classifier(head, x)
     for _ in range(4):                # (found out of date, built, run)
         cache = model.__dict__.get("_nets")
-        if cache is None or cache.mark is None:
-            cache = model.__dict__["_nets"] = Nets(model)
-        key = (x.shape, x.device.index, model.precision)
+        if cache is None or cache.mark is None or (native and cache.classifier not in (None, native)):
+            cache = model.__dict__["_nets"] = Nets(model, head)
+        key = (x.shape, x.device.index, model.precision, native is None)
         net = cache.nets.get(key)
         y = net(x) if net else None
         if not cache.current(model):
             model.__dict__["_nets"] = None
         elif net or net is False or not cache.plain(model):
-            return y if cache.plain(model) else None
+            if y is None or not cache.plain(model):
+                return None
+            return y if native else head(y)
         else:
             with cache.lock, N.building(x.device):
                 if key not in cache.nets:
                     N.make_room(cache.nets, Nets.MOST)
-                    cache.nets[key] = _build(model, x, build)
+                    cache.classifier = native or cache.classifier
+                    cache.nets[key] = _build(model, x, build, head, native is None)
     return None
 
 
-def _build(model, x, build):
+def _build(model, x, build, head, features):
     try:
-        if any(p.device != x.device or p.dtype != torch.float32 for p in model.parameters()):
+        apart = {id(p) for p in head.parameters()}
+        if any(p.device != x.device or p.dtype != torch.float32 for p in model.parameters() if id(p) not in apart):
             return False
         net = N.Net(*x.shape, x.device)
-        net.nchw = model.precision in NCHW_PRECISIONS
+        net.nchw, net.features = model.precision in NCHW_PRECISIONS, features
         return build(model, net, model.precision)
     except (NotExpressible, AttributeError, TypeError, IndexError, KeyError):      # (a module without what the builders read: the layers decide)
         return False

@@ -222,7 +222,7 @@ class TKResNet(nn.Module):
         if not x.is_cuda:
             raise TdcError(ERR_UNSUPPORTED, "TKResNet runs on CUDA tensors only")
         x = x.contiguous().float()
-        y = programs.forward(self, x, programs.build_resnet)
+        y = programs.forward(self, x, programs.build_resnet, self.fc)
         if y is not None:
             return y
         s, b = _fold_bn(self.bn1)

@@ -104,7 +104,7 @@ class TKVGG(nn.Module):
 
     def forward(self, x):
         if x.is_cuda and not self.training:
-            y = programs.forward(self, x.contiguous().float(), programs.build_vgg)
+            y = programs.forward(self, x.contiguous().float(), programs.build_vgg, self.head.fc)
             if y is not None:
                 return y
         x = self.forward_features(x)

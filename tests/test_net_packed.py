@@ -448,3 +448,34 @@ def test_modules_pass_their_range_on(N):
             y = m(torch.randn(2, C, H, H, device="cuda"))
             y.mul_(1e6)                                 # what it carries is no bound any more
             assert rel(m(y), tucker(y)) <= FP32_TOL and tc.status() == 0
+
+
+@pytest.mark.parametrize("B,C,affine", [(1, 64, False), (5, 37, True), (40, 50, False)])
+def test_averages_without_a_classifier(N, B, C, affine):
+    x, w, s, b = draw(9, B, C, C, 7, 5, 1)
+    net = N.Net(B, C, 7, 5, x.device)
+    net.head(net.conv(net.pack(), N.CONV1x1, w, out=N.PLANES), None, None, *((s, b) if affine else (None, None)))
+    ref = F.conv2d(x.double(), w.double())
+    if affine:
+        ref = (ref * s.double().view(1, -1, 1, 1) + b.double().view(1, -1, 1, 1)).relu()
+    assert rel(net.finish((B, C))(x), ref.mean((2, 3))) <= FP32_TOL
+
+
+@pytest.mark.parametrize("net", ["tkc_resnet18", "tkc_densenet121"])
+@pytest.mark.parametrize("precision", ["auto", "fp32"])
+def test_classifier_is_trained_on_a_frozen_network(N, net, precision):
+    """The gradient of the classifier is that of torch's Linear on the network's averages; the logits are those of the net's own."""
+    import tdc_b200 as T
+    m = T.fill_deterministic(getattr(T, net)(precision=precision).eval(), seed=0, gain=0.7 if "dense" in net else 1.0).cuda()
+    fc = m.fc if hasattr(m, "fc") else m.classifier
+    x = torch.randn(2, 3, 96, 64, generator=torch.Generator().manual_seed(2)).cuda()
+    y = m(x)
+    g = torch.randn_like(y)
+    y.backward(g)
+    with torch.no_grad():
+        assert rel(m(x), y.double().detach()) <= FP32_TOL and any(n and not n.features for n in m._nets.nets.values())
+        seen = []
+        h = fc.register_forward_hook(lambda mod, a, out: seen.append(a[0]))
+        m(x)
+        h.remove()
+    assert rel(fc.weight.grad, g.double().t() @ seen[0].double()) <= FP32_TOL and torch.allclose(fc.bias.grad, g.sum(0))

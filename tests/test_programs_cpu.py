@@ -12,7 +12,7 @@ class Steps:
     made = []
 
     def __init__(self, B, C, H, W, device):
-        self.shape, self.device, self.nchw, self.steps = (B, C, H, W), device, False, []
+        self.shape, self.device, self.nchw, self.features, self.steps = (B, C, H, W), device, False, False, []
         Steps.made.append(self)
 
     def _step(self, *what):
@@ -31,8 +31,8 @@ class Steps:
     def pool(self, src, k, stride, pad=0, **kw):
         return self._step("pool", src, k, stride, pad)
 
-    def head(self, src, *a, **kw):
-        return self._step("head", src)
+    def head(self, src, weight=None, *a, **kw):
+        return self._step("head" if weight is not None else "averages", src)
 
     def finish(self, out_shape):
         self.out_shape = tuple(out_shape)
@@ -65,14 +65,14 @@ def make(P, name, **kw):
     T = types.SimpleNamespace(tkc_resnet18=T.tkc_resnet18, tkc_resnet50=T.tkc_resnet50, TKVGG=vgg.TKVGG, TKDenseNet=densenet.TKDenseNet)
     ctor, build, size = nets(T)[name]
     model = ctor(precision="auto", **kw).eval()
-    return model, caller(P, model, build, size)
+
+    def call(B=1, H=size, W=size, channels=3, grad=False):
+        with torch.set_grad_enabled(grad):
+            return P.forward(model, torch.zeros(B, channels, H, W), getattr(P, build), model.get_submodule(HEADS[name]))
+    return model, call
 
 
-def caller(P, model, build, size, channels=3):
-    def call(B=1, H=size, W=size, channels=channels):
-        with torch.no_grad():
-            return P.forward(model, torch.zeros(B, channels, H, W), getattr(P, build))
-    return call
+HEADS = {"resnet18": "fc", "resnet50": "fc", "vgg": "head.fc", "densenet": "classifier"}
 
 
 NAMES = ("resnet18", "resnet50", "vgg", "densenet")
@@ -130,21 +130,76 @@ def test_a_module_that_does_something_else_is_called(P, what, before):
     assert call() is None and call() is None
 
 
-HEADS = {"resnet18": "fc", "vgg": "head.fc", "densenet": "classifier"}
-
-
 @pytest.mark.parametrize("name", sorted(HEADS))
 @pytest.mark.parametrize("head", ["identity", "chain", "subclass"])
 @pytest.mark.parametrize("before", [True, False])
 def test_any_classifier_is_called(P, name, head, before):
+    """The launch of a net stands for nn.Linear; another module is called on the averages."""
     model, call = make(P, name)
     if not before:
-        assert call() is not None
+        assert call() is not None and Steps.made[-1].steps[-1][0] == "head"
     owner, _, leaf = HEADS[name].rpartition(".")
     n = model.get_submodule(HEADS[name]).in_features
     own = {"identity": nn.Identity, "chain": lambda: nn.Sequential(nn.Linear(n, 7)), "subclass": lambda: Scaled(n, 7)}[head]().eval()
     setattr(model.get_submodule(owner), leaf, own)
-    assert call() is None
+    y = call()
+    assert torch.equal(y, own(torch.zeros(1, n))) and Steps.made[-1].steps[-1][0] == "averages"
+
+
+def called(P, monkeypatch, name="resnet18"):
+    """(model, call, the list of the inputs its classifier was called on)"""
+    model, call = make(P, name)
+    seen, forward = [], nn.Linear.forward
+    monkeypatch.setattr(nn.Linear, "forward", lambda self, x: seen.append(x.shape) or forward(self, x))
+    return model, call, seen
+
+
+def test_the_classifier_has_its_gradient(P, monkeypatch):
+    """A frozen network whose classifier is trained: with gradients enabled the classifier is torch's, without them the net's."""
+    model, call, seen = called(P, monkeypatch)
+    y = call(grad=True)
+    y.sum().backward()
+    assert seen == [(1, 512)] and model.fc.weight.grad is not None and torch.equal(model.fc.bias.grad, torch.ones(1000))
+    assert not call().requires_grad and len(seen) == 1
+    model.fc.requires_grad_(False)
+    assert not call(grad=True).requires_grad and len(seen) == 1
+
+
+def test_what_torch_does_around_a_call_reaches_the_classifier(P, monkeypatch):
+    """Autocast, forward-mode derivatives, function transforms, dispatch modes and hooks on the classifier."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    model, call, seen = called(P, monkeypatch)
+    assert call() is not None and not seen
+    with torch.autocast("cpu", dtype=torch.bfloat16):
+        assert call().dtype == torch.bfloat16 and len(seen) == 1
+    with torch.autograd.forward_ad.dual_level():
+        assert call() is not None and len(seen) == 2
+    torch.func.vmap(lambda v: v + call().sum())(torch.zeros(2))
+    assert len(seen) == 3
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, f, types, args=(), kwargs=None):
+            return f(*args, **(kwargs or {}))
+    with Mode():
+        assert call() is not None and len(seen) == 4
+    h = model.fc.register_forward_hook(lambda *a: None)
+    assert call() is not None and len(seen) == 5
+    h.remove()
+    model.fc.train()
+    assert call() is not None and len(seen) == 5
+
+
+def test_a_replaced_classifier_weight_is_read(P):
+    """A net's last launch reads the weight where it lies: written in place it counts at once, replaced it means another net."""
+    model, call = make(P, "resnet18")
+    call()
+    with torch.no_grad():
+        model.fc.weight.mul_(2)
+    call()
+    assert len(Steps.made) == 1
+    model.fc.weight = nn.Parameter(torch.zeros(5, 512))
+    model.fc.bias = None
+    assert call().shape == (1, 5) and len(Steps.made) == 2
 
 
 def test_hooks_on_every_module(P):
