@@ -8,6 +8,7 @@ kernels otherwise.
 """
 from . import ops
 from ._lib import W_CRSK
+from .net import Cache, building
 
 # tensor-core mode of each precision name (tdc_tc_plan.mode)
 MODES = {"tf32": 1, "tf32x3": 3, "fp16x3": 4}
@@ -42,11 +43,10 @@ def one_conv(owner, name, x, w_kcrs, w_crsk, scale, shift, residual, relu, strid
 
 def channel_last(owner, name, w):
     """[C][R][S][K] copy of a filter, kept on the module that owns it until the filter is written to or replaced."""
-    store = owner.__dict__.setdefault("_channel_last", {})
+    store = owner.__dict__.setdefault("_channel_last", Cache())
     key = (w._version, w.data_ptr())
     hit = store.get(name)
     if hit is None or hit[0] != key:
-        from .net import building
         with building(w.device):
             w = w.detach().contiguous()
             hit = store[name] = (key, ops.permute_weights(w), w)      # (the filter itself too: its address is the key)

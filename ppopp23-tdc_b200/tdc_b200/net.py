@@ -70,8 +70,8 @@ def make_room(table, most):
 
 
 class Cache(dict):
-    """Nets kept on an object that may be copied or pickled: a net is a handle to memory of this process, so a copy starts
-    without them."""
+    """Nets and prepared memory kept on an object that may be copied or pickled.  A net is a handle to memory of this process, and what
+    is kept under the addresses of tensors says nothing about another object's or process's: a copy starts without them."""
 
     def __deepcopy__(self, memo):
         return Cache()
@@ -141,7 +141,7 @@ class Net:
         return t.value if into >= 0 or out == NCHW else self._made(t.value, K)
 
     def _filter(self, kind, weight, nt, nbytes, scale, bias, owner, name):
-        store = owner.__dict__.setdefault("_net_filters", {}) if owner is not None else {}
+        store = owner.__dict__.setdefault("_net_filters", Cache()) if owner is not None else {}
         at, key = (name, kind, nt, scale is None, bias is None), _key(weight, scale, bias)
         hit = store.get(at)
         if hit is None or hit[0] != key:

@@ -48,7 +48,8 @@ def fold_bn(bn):
     """(scale, shift, {max |scale|, max |shift|}) of an inference BatchNorm on the GPU, kept on the module until one of its
     tensors changes."""
     key = (bn.eps,) + N._key(bn.running_var, bn.running_mean, bn.weight, bn.bias)
-    hit = bn.__dict__.get("_tdc_fold")
+    kept = bn.__dict__.setdefault("_tdc_fold", N.Cache())
+    hit = kept.get("fold")
     if hit is None or hit[0] != key:
         n, dev = bn.running_var.numel(), bn.running_var.device
         n4 = (n + 3) // 4 * 4                                 # scale and shift 16-byte aligned
@@ -57,7 +58,7 @@ def fold_bn(bn):
         with N.building(dev):
             check(lib.tdc_net_fold_bn(bn.running_var.data_ptr(), bn.running_mean.data_ptr(), bn.weight.data_ptr() if bn.weight is not None else None,
                                       bn.bias.data_ptr() if bn.bias is not None else None, bn.eps, n, scale.data_ptr(), shift.data_ptr(), bound.data_ptr(), _stream()))
-        hit = bn.__dict__["_tdc_fold"] = (key, scale, shift, bound)
+        hit = kept["fold"] = (key, scale, shift, bound)
     return hit[1:]
 
 
@@ -124,10 +125,11 @@ def _with_bias(conv, scale, shift):
     if scale is None and shift is None:
         return conv.bias.detach()
     key = N._key(conv.bias, scale, shift)
-    hit = conv.__dict__.get("_tdc_shift")
+    kept = conv.__dict__.setdefault("_tdc_shift", N.Cache())
+    hit = kept.get("shift")
     if hit is None or hit[0] != key:
         b = conv.bias.detach() if scale is None else conv.bias.detach() * scale
-        hit = conv.__dict__["_tdc_shift"] = (key, b if shift is None else shift + b, conv.bias.detach(), scale, shift)
+        hit = kept["shift"] = (key, b if shift is None else shift + b, conv.bias.detach(), scale, shift)
     return hit[1]
 
 

@@ -377,3 +377,25 @@ def test_range_of_a_tensor_ends_when_it_is_written_to():
         z = torch.zeros(4)
         ops.leave_range(z, bound)
         assert ops.range_of(z) is bound
+
+
+def test_copies_start_without_what_is_kept_by_address(built, monkeypatch):
+    """A copied or loaded module's tensors may lie where the original's did, with the same version."""
+    import copy
+    import pickle
+    from tdc_b200 import dispatch, net, programs
+    monkeypatch.setattr(programs, "lib", types.SimpleNamespace(tdc_net_fold_bn=lambda *a: 0))
+    monkeypatch.setattr(net, "lib", types.SimpleNamespace(tdc_net_filter_prepare=lambda *a: 0))
+    monkeypatch.setattr(dispatch.ops, "permute_weights", lambda w: w.permute(1, 2, 3, 0).contiguous())
+    monkeypatch.setattr(net, "_dev_f32", lambda t, name: t.data_ptr())
+    for m in (programs, net):
+        monkeypatch.setattr(m, "_stream", lambda: 0)
+    conv, bn = nn.Conv2d(4, 8, 1), nn.BatchNorm2d(8).eval()
+    programs.fold_bn(bn)
+    programs._with_bias(conv, torch.rand(8), torch.rand(8))
+    dispatch.channel_last(conv, "weight", conv.weight)
+    net.Net._filter(None, net.CONV1x1, conv.weight, 32, 64, None, None, conv, "weight")
+    kept = {"_tdc_fold": bn, "_tdc_shift": conv, "_channel_last": conv, "_net_filters": conv}
+    assert all(m.__dict__[name] for name, m in kept.items())
+    for again in (copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))):
+        assert not any(again(m).__dict__[name] for name, m in kept.items())
