@@ -51,13 +51,21 @@ def fold_bn(bn):
     kept = bn.__dict__.setdefault("_tdc_fold", N.Cache())
     hit = kept.get("fold")
     if hit is None or hit[0] != key:
+        tensors = (bn.running_var, bn.running_mean, bn.weight, bn.bias)
         n, dev = bn.running_var.numel(), bn.running_var.device
         n4 = (n + 3) // 4 * 4                                 # scale and shift 16-byte aligned
         buf = torch.empty(2 * n4 + 2, device=dev, dtype=torch.float32)
         scale, shift, bound = buf[:n], buf[n4:n4 + n], buf[2 * n4:]
         with N.building(dev):
-            check(lib.tdc_net_fold_bn(bn.running_var.data_ptr(), bn.running_mean.data_ptr(), bn.weight.data_ptr() if bn.weight is not None else None,
-                                      bn.bias.data_ptr() if bn.bias is not None else None, bn.eps, n, scale.data_ptr(), shift.data_ptr(), bound.data_ptr(), _stream()))
+            if all(t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.device == dev and t.numel() == n) for t in tensors):
+                var, mean, g, b = (None if t is None else t.data_ptr() for t in tensors)
+                check(lib.tdc_net_fold_bn(var, mean, g, b, bn.eps, n, scale.data_ptr(), shift.data_ptr(), bound.data_ptr(), _stream()))
+            else:                                             # another type or layout: the same arithmetic
+                with torch.no_grad():
+                    var, mean = bn.running_var.double(), bn.running_mean.double()
+                    s = (1.0 if bn.weight is None else bn.weight.double()) / torch.sqrt(var + bn.eps)
+                    scale.copy_(s), shift.copy_((0.0 if bn.bias is None else bn.bias.double()) - mean * s)
+                    bound.copy_(torch.stack([scale.abs().max(), shift.abs().max()]))
         hit = kept["fold"] = (key, scale, shift, bound)
     return hit[1:]
 

@@ -399,3 +399,19 @@ def test_copies_start_without_what_is_kept_by_address(built, monkeypatch):
     assert all(m.__dict__[name] for name, m in kept.items())
     for again in (copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))):
         assert not any(again(m).__dict__[name] for name, m in kept.items())
+
+
+@pytest.mark.parametrize("what", ["double", "strided", "no affine"])
+def test_folded_batchnorm_of_other_types_and_layouts(built, monkeypatch, what):
+    """The library's fold reads fp32 values that lie next to each other; statistics of another type or layout are not handed to it."""
+    from tdc_b200 import programs
+    monkeypatch.setattr(programs, "lib", types.SimpleNamespace(tdc_net_fold_bn=lambda *a: pytest.fail("called")))
+    bn = nn.BatchNorm2d(8, affine=what != "no affine").eval()
+    bn.running_var, bn.running_mean = torch.rand(8).double() + 0.5, torch.randn(8).double()
+    if what == "strided":
+        bn.running_var, bn.running_mean = (torch.rand(8, 3) + 0.5)[:, 1], torch.randn(8)
+    scale, shift, bound = programs.fold_bn(bn)
+    g, b = (1.0, 0.0) if bn.weight is None else (bn.weight.detach().double(), bn.bias.detach().double())
+    s = g / (bn.running_var.double() + bn.eps).sqrt()
+    assert torch.equal(scale, s.float()) and torch.equal(shift, (b - bn.running_mean.double() * s).float())
+    assert bound.tolist() == [float(scale.abs().max()), float(shift.abs().max())]
