@@ -377,6 +377,14 @@ __device__ __forceinline__ void pool_columns(const f2 (&p)[8], int odd, float (&
     }
 }
 
+// Waits (bounded) for the copies of every stage, by what the producer left: the next stage and its phase.  Stages never used pass at
+// once.
+__device__ __forceinline__ void copies_landed(uint64_t* full_bar, int ns, unsigned int left) {
+    const int st = (int)(left & 255u);
+    const uint32_t use = left >> 8 & 1u;
+    for (int s = 0; s < ns; ++s) mbar_wait(&full_bar[s], s < st ? use : use ^ 1u);
+}
+
 // POOL: the epilogue also does the max pooling that follows.  The feature map of full size — the largest tensor of the network
 // at a stem or between VGG's first stages — is then never written nor read back, and the epilogue splits and stores a quarter of
 // the values.  Rows meet in registers (the two position tiles are two rows; a 3x3 window's third row stays from the tile before),
@@ -392,7 +400,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) conv_pk_kernel(const __grid_con
     uint64_t* wfull_bar = tempty_bar + 8;                                 // [groups of a tile] the resident filter blocks of a stage have landed
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wfull_bar + PK_MAXRES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    unsigned int* words = tmem_slot + 2;                                  // [0] max|x|, [1] max|residual|, [2] max|y| of this CTA
+    unsigned int* words = tmem_slot + 2;                                  // [0] max|x|, [2] max|y| of this CTA, [3] what the producer has asked for
     float* s_scale = reinterpret_cast<float*>(smem_raw + PK_HEADER);
     float* s_bias = s_scale + a.s_floats;
     float* edge = s_bias + a.s_floats;                                    // POOL_3x3: [2][group][warp][2][8] right columns of a warp's last pair
@@ -465,11 +473,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) conv_pk_kernel(const __grid_con
                 }
                 if (!ok) break;
             }
-            // leaving early: no copy of this CTA may still be in flight when it exits (stages never used pass at once)
-            if (*abort_flag) {
-                for (int s = 0; s < a.ns; ++s) mbar_wait(&full_bar[s], (uint32_t)(s < st ? use : use ^ 1));
-                for (int g = 0; g < loaded; ++g) mbar_wait(&wfull_bar[g], 0);
-            }
+            words[3] = (unsigned int)(st | use << 8 | loaded << 9);
         }
         __syncwarp();
     } else if (warp < PK_EW0) {
@@ -657,7 +661,12 @@ __global__ void __launch_bounds__(PK_THREADS, 1) conv_pk_kernel(const __grid_con
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (tid == 0) {
-        if (*abort_flag && a.status) atomicCAS(a.status, 0, 1);
+        if (*abort_flag) {
+            if (a.status) atomicCAS(a.status, 0, 1);
+            // leaving early, whoever gave up: no copy of this CTA may still be in flight when it exits
+            copies_landed(full_bar, a.ns, words[3]);
+            for (int g = 0; g < (int)(words[3] >> 9); ++g) mbar_wait(&wfull_bar[g], 0);
+        }
         if (a.status && words[2] >= 0x7f800000u) atomicCAS(a.status, 0, 2);      // an output that is not finite
         leave_max(a, words[2]);
     }
@@ -755,8 +764,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 2) conv_pk_split_kernel(const _
                 patch(kb0, st);
                 if (++st == a.ns) { st = 0; use ^= 1; }
             }
-            if (*abort_flag)
-                for (int s = 0; s < a.ns; ++s) mbar_wait(&full_bar[s], (uint32_t)(s < st ? use : use ^ 1));
+            words[4] = (unsigned int)(st | use << 8);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -882,8 +890,21 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 2) conv_pk_split_kernel(const _
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*abort_flag) {                                                    // (uniform: nobody writes it behind the barrier)
+        if (tid == 0) {
+            if (a.status) atomicCAS(a.status, 0, 1);
+            copies_landed(full_bar, a.ns, words[4]);
+        }
+        // The others of the cluster may still be sending to this CTA: it leaves when they have sent (or have left themselves; their
+        // waits are bounded like these) and what they sent has landed.
+        if (ks > 1) {
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            if (tid == 0) mbar_wait(xfull_bar, 0);
+        }
+    }
     if (tid == 0) {
-        if (*abort_flag && a.status) atomicCAS(a.status, 0, 1);
         if (a.status && words[2] >= 0x7f800000u) atomicCAS(a.status, 0, 2);
         leave_max(a, words[2]);
     }
