@@ -129,6 +129,14 @@ class TcConv:
         B, Cc, H, W = x.shape
         if kind is None or self.R != self.S or (padding is not None and padding != self.R // 2):
             return None
+        # (what the one launch refuses stays refused, by it)
+        if not self.general and stride > 1 and self.R != 1:
+            return None
+        rows = (stride, padding & 1) if self.general and strided_rows(self.S, stride) else None
+        plan = self._make_plan(self.plan.nt, rows) if rows else self.plan
+        flags = (stride - 1) | (padding << 4 if self.general else 0)
+        if lib.tdc_tc_check_launch(C.byref(plan), B, H, W, flags) in (_lib.ERR_UNSUPPORTED, _lib.ERR_SHAPE):
+            return None
         if kind == N.CONV3x3 and 3 * Cc <= 16:
             kind, pack = N.CONV3x3_ROWS, N.PACK_ROWS
         if self.packed is None and (_TUNING or not self._packs(kind, B, Cc, H, W, stride)):

@@ -479,3 +479,22 @@ def test_classifier_is_trained_on_a_frozen_network(N, net, precision):
         m(x)
         h.remove()
     assert rel(fc.weight.grad, g.double().t() @ seen[0].double()) <= FP32_TOL and torch.allclose(fc.bias.grad, g.sum(0))
+
+
+@pytest.mark.parametrize("R,general,kw,H,W", [(3, False, {"stride": 2}, 12, 12), (3, False, {}, 4, 300), (1, False, {}, 4, 300), (3, True, {"stride": 2, "padding": 1}, 4, 600)])
+def test_packed_form_takes_no_call_the_layer_refuses(N, monkeypatch, R, general, kw, H, W):
+    """A stride without a general plan, an image wider than a plan's 256 positions."""
+    import tdc_b200 as T
+    from tdc_b200 import tc
+    monkeypatch.setattr(tc, "_TUNING", False)
+    x, w, _, _ = draw(24, 1, 16, 24, H, W, R)
+    codes = []
+    for packed in (False, True, None):
+        conv = T.TcConv(w, mode=4, general=general)
+        conv.packed = packed
+        try:
+            conv(x, **kw)
+            codes.append(0)
+        except T.TdcError as e:
+            codes.append(e.code)
+    assert codes[0] == codes[1] == codes[2] and codes[0] in (0, 2, 3, 5)
