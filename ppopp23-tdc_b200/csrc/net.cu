@@ -57,7 +57,8 @@ int opt_in(const void* fn, int smem_max) {
     return e == cudaSuccess ? TDC_OK : fail(TDC_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
 }
 
-cudaError_t launch(const void* fn, dim3 grid, int threads, int cluster, size_t smem, void* args, cudaStream_t st) {
+// A tdc_status; the steps that call other entry points return theirs.
+int launch(const void* fn, dim3 grid, int threads, int cluster, size_t smem, void* args, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -67,7 +68,8 @@ cudaError_t launch(const void* fn, dim3 grid, int threads, int cluster, size_t s
     attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
     void* argv[] = {args};
-    return cudaLaunchKernelExC(&cfg, fn, argv);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, argv);
+    return e == cudaSuccess ? TDC_OK : fail(TDC_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
 }
 
 struct Buffer { size_t bytes = 0, off = 0; int def = -1, last = -1; };
@@ -95,7 +97,7 @@ struct tdc_net {
     int B = 0, C = 0, H = 0, W = 0;    // the NCHW input
     std::vector<Tensor> tensors;
     std::vector<Buffer> buffers;
-    std::vector<std::function<cudaError_t(const RunArgs&)>> ops;
+    std::vector<std::function<int(const RunArgs&)>> ops;
     size_t meta_floats = 0, meta_off = 0, arena_bytes = 0;
     bool finished = false, packed_y = false;        // packed_y: a convolution on packed activations writes y
 
@@ -493,9 +495,6 @@ static int nchw_dims(const tdc_net* n, int src, int* C, int* H, int* W) {
     return TDC_OK;
 }
 
-// The kernels report failures in their own words; a net's run stops at the first one.
-static cudaError_t step_result(int rc) { return rc == TDC_OK ? cudaSuccess : cudaErrorUnknown; }
-
 int tdc_net_nchw_conv(tdc_net* n, int src, const tdc_net_nchw* d, int* out) {
     if (!n || !d || !out || !d->filter) return fail(TDC_ERR_NULL, "net, conv, filter and out must be non-NULL");
     int C, H, W;
@@ -518,11 +517,11 @@ int tdc_net_nchw_conv(tdc_net* n, int src, const tdc_net_nchw* d, int* out) {
         const tdc_epilogue e{a.scale, a.bias, a.residual >= 0 ? n->nchw_at(r, a.residual) : nullptr, a.relu};
         float* y = to_y ? r.y : const_cast<float*>(n->nchw_at(r, id));
         if (tc && plan.mode == 4)          // (the maxima of one step's output are the range of the next one's input)
-            return step_result(tdc_conv2d_tc_ranged(&plan, n->nchw_at(r, src), a.filter, y, n->B, H, W, &e, a.flags, src < 0 ? r.x_absmax : n->range_at(r, src),
-                                                    to_y ? r.y_absmax : n->range_at(r, id), r.st));
-        if (tc) return step_result(tdc_conv2d_tc(&plan, n->nchw_at(r, src), a.filter, y, n->B, H, W, &e, a.flags, r.st));
-        return step_result(tdc_conv2d_epi_f32(n->nchw_at(r, src), static_cast<const float*>(a.filter), y, n->B, C, H, W, a.K, a.R, a.S, a.pad, a.stride,
-                                              TDC_W_CRSK, &e, nullptr, r.st));
+            return tdc_conv2d_tc_ranged(&plan, n->nchw_at(r, src), a.filter, y, n->B, H, W, &e, a.flags, src < 0 ? r.x_absmax : n->range_at(r, src),
+                                                    to_y ? r.y_absmax : n->range_at(r, id), r.st);
+        if (tc) return tdc_conv2d_tc(&plan, n->nchw_at(r, src), a.filter, y, n->B, H, W, &e, a.flags, r.st);
+        return tdc_conv2d_epi_f32(n->nchw_at(r, src), static_cast<const float*>(a.filter), y, n->B, C, H, W, a.K, a.R, a.S, a.pad, a.stride,
+                                              TDC_W_CRSK, &e, nullptr, r.st);
     });
     *out = id;
     return TDC_OK;
@@ -537,7 +536,7 @@ int tdc_net_nchw_pool(tdc_net* n, int src, int k, int stride, int pad, int mode,
     n->use_nchw(src);
     const int id = n->nchw_tensor(C, (H - k + 2 * pad) / stride + 1, (W - k + 2 * pad) / stride + 1);
     n->ops.push_back([n, src, id, C, H, W, k, stride, pad, mode](const RunArgs& r) {
-        return step_result(tdc_pool2d_f32(n->nchw_at(r, src), const_cast<float*>(n->nchw_at(r, id)), n->B, C, H, W, k, k, pad, stride, mode, r.st));
+        return tdc_pool2d_f32(n->nchw_at(r, src), const_cast<float*>(n->nchw_at(r, id)), n->B, C, H, W, k, k, pad, stride, mode, r.st);
     });
     *out = id;
     return TDC_OK;
@@ -568,7 +567,7 @@ int tdc_net_nchw_affine(tdc_net* n, int src, int channels, const float* scale, c
     const int c0 = into < 0 ? 0 : into_c;
     const long long xs = (long long)C * H * W, ys = (long long)n->tensors[id].C * H * W;
     n->ops.push_back([n, src, id, c, c0, H, W, xs, ys, scale, shift, relu](const RunArgs& r) {
-        return step_result(tdc_affine_relu_f32(n->nchw_at(r, src), const_cast<float*>(n->nchw_at(r, id)) + (long long)c0 * H * W, scale, shift, n->B, c, H * W, xs, ys, relu, r.st));
+        return tdc_affine_relu_f32(n->nchw_at(r, src), const_cast<float*>(n->nchw_at(r, id)) + (long long)c0 * H * W, scale, shift, n->B, c, H * W, xs, ys, relu, r.st);
     });
     *out = id;
     return TDC_OK;
@@ -654,9 +653,8 @@ static int run(const tdc_net* n, RunArgs r, size_t arena_bytes) {
     if (reinterpret_cast<uintptr_t>(r.arena) % 16) return fail(TDC_ERR_UNSUPPORTED, "the arena is 16-byte aligned");
     const OnDevice here(n->device);
     for (const auto& op : n->ops) {
-        const cudaError_t e = op(r);
-        if (e == cudaErrorUnknown) return TDC_ERR_CUDA;           // a step's entry point has said why
-        if (e != cudaSuccess) return fail(TDC_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+        const int rc = op(r);
+        if (rc) return rc;               // the step has said why
     }
     return TDC_OK;
 }

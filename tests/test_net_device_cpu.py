@@ -1,5 +1,5 @@
-"""A net does its work on the device that was current when it was made, whichever is current later: the library against a CUDA
-runtime that only keeps book of devices and launches (no GPU)."""
+"""A net does its work on the device that was current when it was made, whichever is current later, and its run's status is that of
+the step that failed: the library against a CUDA runtime that only keeps book of devices and launches (no GPU)."""
 import os
 import subprocess
 
@@ -45,6 +45,14 @@ int main() {
     MUST(tdc_net_run(n, x, nullptr, y, nullptr, arena, bytes, nullptr));
     printf("opened %d %d launches %d %d current %d\n", opened[0], opened[1], launches[0], launches[1], current);
     tdc_net_destroy(n);
+    // a step that its entry point refuses: the run's status is that refusal
+    MUST(tdc_net_create(&n, 1, 16, 8, 8));
+    tdc_net_nchw c{};
+    c.K = 8; c.R = c.S = 1; c.stride = 3; c.filter = w; c.residual = -1; c.to_y = 1;
+    MUST(tdc_net_nchw_conv(n, -1, &c, &t));
+    MUST(tdc_net_finish(n, &bytes));
+    const int rc = tdc_net_run(n, x, nullptr, y, nullptr, x, bytes, nullptr);
+    printf("status %d %s\n", rc, tdc_last_error_string());
     return 0;
 }
 """
@@ -60,7 +68,9 @@ def test_the_device_of_a_net(built, tmp_path):
     r = subprocess.run(["nvcc", "-std=c++17", "-cudart", "shared", "-I", os.path.join(ROOT, "include"), "-o", exe, str(src), *objs, "-Xlinker", "--allow-multiple-definition"], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     r = subprocess.run([exe], capture_output=True, text=True)
-    assert r.returncode == 0 and r.stdout.split("\n")[0] == "opened 0 2 launches 0 4 current 0", r.stdout + r.stderr
+    lines = r.stdout.split("\n")
+    assert r.returncode == 0 and lines[0] == "opened 0 2 launches 0 4 current 0", r.stdout + r.stderr
+    assert lines[1].startswith("status 3 stride 3"), r.stdout
 
 
 def test_images_whose_positions_do_not_count_in_32_bits_are_refused(built):
