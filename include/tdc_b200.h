@@ -439,7 +439,9 @@ TDC_API void tdc_tkconv_destroy(tdc_tkconv* l);
  * (A100-evaluation/EndToEnd/resnet18-tk/src/main.cu:127-155). */
 typedef struct tdc_net tdc_net;
 
-/* What tdc_net_pack, the first step of a net, makes of the NCHW input. */
+/* What tdc_net_pack, the first step of a net, makes of the NCHW input.  Its scale comes from the maxima a run is given, else from the true
+ * maximum of an input of up to 2^18 values and from a sample of a larger one, with tdc_conv2d_tc_ranged's headroom of 256; a value
+ * beyond makes outputs that are not finite and sets the status word to 2. */
 #define TDC_NET_PACK       0   /* channels and positions as they are */
 #define TDC_NET_PACK_SPLIT 1   /* positions by (row parity, column parity): what stride-2 convolutions read */
 #define TDC_NET_PACK_S2D   2   /* for TDC_NET_CONV7x7_S2 */

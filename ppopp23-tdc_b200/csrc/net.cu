@@ -269,18 +269,21 @@ int tdc_net_pack(tdc_net* n, int kind, int* out) {
     PackArgs a{};
     a.B = n->B; a.C = n->C; a.H = n->H; a.W = n->W;
     a.groups = t.groups; a.front = space_front(s); a.d = s; a.y_plane = tdc_net::pk_plane(t); a.status = n->f.status;
-    const unsigned grid = blocks_for(items, n->f);
+    const bool exact = (long long)n->B * n->C * n->H * n->W <= PACK_EXACT;
+    unsigned grid = blocks_for(items, n->f);
+    if (exact) grid = std::min<unsigned>((grid + PACK_CLUSTER - 1) / PACK_CLUSTER, PACK_SLOTS / PACK_CLUSTER) * PACK_CLUSTER;
     t.slots = (int)grid;
-    const void* fn = kind == PACK_SAME ? (const void*)&pack_kernel<PACK_SAME> : kind == PACK_SPLIT ? (const void*)&pack_kernel<PACK_SPLIT>
-                   : kind == PACK_S2D ? (const void*)&pack_kernel<PACK_S2D> : (const void*)&pack_kernel<PACK_ROW3>;
-    n->ops.push_back([n, id, a, grid, fn](const RunArgs& r) {
+    const void* const forms[2][4] = {{(const void*)&pack_kernel<PACK_SAME, false>, (const void*)&pack_kernel<PACK_SPLIT, false>, (const void*)&pack_kernel<PACK_S2D, false>, (const void*)&pack_kernel<PACK_ROW3, false>},
+                                     {(const void*)&pack_kernel<PACK_SAME, true>, (const void*)&pack_kernel<PACK_SPLIT, true>, (const void*)&pack_kernel<PACK_S2D, true>, (const void*)&pack_kernel<PACK_ROW3, true>}};
+    const void* fn = forms[exact][kind];
+    n->ops.push_back([n, id, a, grid, fn, exact](const RunArgs& r) {
         PackArgs p = a;
         const Tensor& t = n->tensors[id];
         p.x = r.x; p.absmax = r.x_absmax; p.absmax_n = tdc_tc::ABSMAX_SLOTS;
         p.y = n->pk_at(r, t);
         p.y_scale = n->meta_at(r, t); p.y_slots = p.y_scale + 1;
         p.zero = p.y_slots + PACK_SLOTS; p.zeros = (int)n->meta_floats - (1 + PACK_SLOTS);
-        return launch(fn, dim3(grid), OPS_THREADS, 1, 0, &p, r.st);
+        return launch(fn, dim3(grid), OPS_THREADS, exact ? PACK_CLUSTER : 1, 0, &p, r.st);
     });
     *out = id;
     return TDC_OK;

@@ -48,17 +48,56 @@ struct PackArgs {
 //   ROW3   channel 3 c + dx holds column x + dx - 1: a 3x3 filter over few channels is three row taps on these, one channel
 //          block where the plain form takes nine taps of a block that is mostly zeros.
 // Bound by memory: 4 bytes read and 4 written per value.
-template <int KIND>
+//
+// EXACT: launched in clusters of PACK_CLUSTER, each of which finds the true maximum of x for itself, every CTA of a share of it;
+// the second reading comes out of cache.  For inputs of up to PACK_EXACT values that costs about what the round trip of the sample does,
+// and layers of that size ran on fp32 arithmetic, which has no range, before they ran on packed operands.
+constexpr int PACK_CLUSTER = 8;
+constexpr long long PACK_EXACT = 1 << 18;
+
+// Largest magnitude of x[0, n), by the cluster; every thread gets it.
+__device__ __forceinline__ unsigned int cluster_absmax(const float* x, long long n, unsigned int* word, unsigned int* peers) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // every CTA runs before its shared memory is written to
+    uint32_t rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int first = (int)rank * OPS_THREADS + (int)threadIdx.x;
+    constexpr int STEP = PACK_CLUSTER * OPS_THREADS;
+    unsigned int m = 0;
+    auto take = [&](float v) { m = max(m, __float_as_uint(v) & 0x7fffffffu); };
+    const int n4 = reinterpret_cast<uintptr_t>(x) % 16 == 0 ? (int)(n / 4) : 0;      // (n is at most PACK_EXACT)
+#pragma unroll 8
+    for (int i = first; i < n4; i += STEP) {
+        const float4 v = reinterpret_cast<const float4*>(x)[i];
+        take(v.x); take(v.y); take(v.z); take(v.w);
+    }
+#pragma unroll 4
+    for (int i = 4 * n4 + first; i < (int)n; i += STEP) take(x[i]);
+    m = block_max(m, word);
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (threadIdx.x < PACK_CLUSTER) {
+        uint32_t dst;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(peers + rank)), "r"(threadIdx.x));
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(m) : "memory");
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int k = 0; k < PACK_CLUSTER; ++k) m = max(m, peers[k]);
+    return m;
+}
+
+template <int KIND, bool EXACT>
 __global__ void __launch_bounds__(OPS_THREADS, 2) pack_kernel(const PackArgs a) {
-    __shared__ unsigned int word;
+    __shared__ unsigned int word, peers[PACK_CLUSTER];
     pdl_enter();
-    // the power of two the values are stored at: from the given maxima, or from 1536 values spread over x, which leaves a
+    // the power of two the values are stored at: from the given maxima, the true one, or from 1536 values spread over x, which leaves a
     // factor of 256 for what the sample missed (what lies beyond is reported: the true maximum is known at the end, and the
     // convolution's outputs are NaN).  One value of each 1536th of x, at an offset that goes round by the golden ratio: at a fixed
     // offset a batch of 16 images of 3 x 224 x 224 was sampled in one column.
     const long long n = (long long)a.B * a.C * a.H * a.W;
     unsigned int m = 0;
     if (a.absmax) m = slots_max(a.absmax, a.absmax_n, threadIdx.x, OPS_THREADS);
+    else if (EXACT) m = cluster_absmax(a.x, n, &word, peers);
     else {
         constexpr unsigned long long PARTS = 3 * OPS_THREADS;
 #pragma unroll
@@ -68,7 +107,7 @@ __global__ void __launch_bounds__(OPS_THREADS, 2) pack_kernel(const PackArgs a) 
             m = max(m, __float_as_uint(a.x[k]) & 0x7fffffffu);
         }
     }
-    const float s = range_scale(__uint_as_float(block_max(m, &word)), a.absmax ? 14 : 8);
+    const float s = range_scale(__uint_as_float(block_max(m, &word)), a.absmax || EXACT ? 14 : 8);
     const uint32_t span = (uint32_t)(a.front + a.d.total), items = span * (uint32_t)a.groups, stride = gridDim.x * OPS_THREADS;
     const int HW = a.H * a.W;                      // (the host keeps an image's plane below 2^31)
     // the 8 values of item i, zeros where it is padding

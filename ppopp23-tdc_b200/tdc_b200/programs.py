@@ -654,6 +654,21 @@ def _one_launch_wins(module, x):
     return direct <= max(13.3, packed)          # (the host time of a call that packs: TcConv._packs)
 
 
+EXACT_RANGE = 1 << 18      # values up to which packing finds the true maximum (csrc/pk_ops.cuh: PACK_EXACT); above, it samples
+
+
+def _has_no_range(module, x):
+    """A module whose layer-by-layer form begins in fp32 arithmetic takes any input; on packed operands that holds where the true maximum
+    is found."""
+    from . import dispatch as D
+    B, Cc, H, W = x.shape
+    if x.numel() <= EXACT_RANGE:
+        return False
+    if D.tucker_strategy(module, x, "auto") == "dense":
+        return not D._on_tensor_cores(B, Cc, module.out_channels, H, W, 3, 3, module.stride[0], 1)
+    return not D._on_tensor_cores(B, Cc, module.in_rank, H, W, 1, 1, 1, 0)
+
+
 def _build_layer(module, x):
     from . import dispatch, tc
     try:
@@ -673,7 +688,10 @@ def _build_layer(module, x):
         stride = _square(module, 3)
         net = N.Net(B, Cc, H, W, x.device)
         K, shape = module.out_channels, (B, module.out_channels, -(-H // stride), -(-W // stride))
-        if not (stride == 1 and module.precision == "auto" and _one_launch_wins(module, x)):
+        unpacked = module.precision == "auto" and (_has_no_range(module, x) or (stride == 1 and _one_launch_wins(module, x)))
+        if unpacked and stride == 2:
+            return False
+        if not unpacked:
             at = At(net.pack(N.PACK_SPLIT if stride == 2 else N.PACK), Cc, H, W, stride == 2)
             conv(net, module, at, None, None, False, module.precision, out=N.NCHW)
             return net.finish(shape)

@@ -309,17 +309,17 @@ assert not bool(conv(x, relu=True)[1].isfinite().all())
 """
 
 
-@pytest.mark.parametrize("case", [(1, 3, 0, 0, (64, 2, 0), 16, 64, 20, 20), (1, 3, 0, 0, (32, 1, 4), 64, 40, 12, 12), (0, 1, 0, 0, (32, 1, 1), 16, 32, 12, 12),
-                                  (1, 3, 0, 2, (64, 2, 0), 16, 64, 20, 20), (3, 7, 2, 3, (64, 2, 0), 3, 64, 40, 40), (4, 3, 3, 0, (64, 1, 0), 3, 64, 40, 40)])
+@pytest.mark.parametrize("case", [(1, 3, 0, 0, (64, 2, 0), 32, 64, 72, 72), (1, 3, 0, 0, (32, 1, 4), 512, 32, 24, 24), (0, 1, 0, 0, (32, 1, 1), 64, 32, 50, 50),
+                                  (1, 3, 0, 2, (64, 2, 0), 32, 64, 72, 72), (3, 7, 2, 3, (64, 2, 0), 3, 64, 240, 240), (4, 3, 3, 0, (64, 1, 0), 3, 64, 240, 240)])
 def test_overflow_is_reported_behind_relu_and_pooling(N, case):
-    """A value beyond 256 times the sampled maximum: the outputs that read it are not finite, ReLU and maxima included, and the status
+    """A value beyond 256 times the sampled maximum (inputs of more than 2^18 values are sampled): the outputs that read it are not finite, ReLU and maxima included, and the status
     word says 2 (in a process of its own, because the word keeps its first report)."""
     r = subprocess.run([sys.executable, "-c", OVERFLOW, os.path.join(ROOT, "ppopp23-tdc_b200"), ROOT, repr(case)], capture_output=True, text=True,
                        env=dict(os.environ, TDC_TC_TUNING="0"), timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
 
 
-@pytest.mark.parametrize("B,C,H,W", [(16, 3, 224, 224), (2, 16, 12, 125)])
+@pytest.mark.parametrize("B,C,H,W", [(16, 3, 224, 224), (2, 16, 100, 125)])
 def test_range_sample_is_spread(N, B, C, H, W):
     """Values at a fixed distance would all lie in the first columns of a batch of 16 images (and in the first image of a small batch),
     which are a thousandth of the rest here: the sample has to see the others."""
@@ -430,7 +430,7 @@ def test_modules_pass_their_range_on(N):
     class HP:
         ranks = {"l": [16, 16]}
     torch.manual_seed(6)
-    C, H = 32, 40
+    C, H = 32, 80
     first = T.TcConv(torch.randn(C, C, 1, 1, device="cuda"), mode=4, exact_range=True)
     for precision in ("auto", "fp16x3"):
         m = T.TKConv2dC_B200(C, C, 3, padding=1, bias=False, hp_dict=HP, name="l").cuda()
@@ -444,7 +444,7 @@ def test_modules_pass_their_range_on(N):
             y = first(x)
             z = m(m(y))
             assert rel(z, tucker(tucker(y))) <= FP32_TOL and tc.status() == 0
-            assert float(z._tdc_absmax.max()) == float(z.abs().max())
+            assert precision == "auto" or float(z._tdc_absmax.max()) == float(z.abs().max())      # ("auto" ends in fp32 here)
             y = m(torch.randn(2, C, H, H, device="cuda"))
             y.mul_(1e6)                                 # what it carries is no bound any more
             assert rel(m(y), tucker(y)) <= FP32_TOL and tc.status() == 0
@@ -498,3 +498,46 @@ def test_packed_form_takes_no_call_the_layer_refuses(N, monkeypatch, R, general,
         except T.TdcError as e:
             codes.append(e.code)
     assert codes[0] == codes[1] == codes[2] and codes[0] in (0, 2, 3, 5)
+
+
+@pytest.mark.parametrize("pack", [0, 1, 2, 3])
+@pytest.mark.parametrize("B,C,H,W", [(1, 3, 17, 19), (2, 20, 33, 40), (1, 64, 64, 64), (5, 1, 200, 250), (1, 5, 3, 3)])
+def test_small_inputs_have_their_true_range(N, pack, B, C, H, W):
+    """Up to 2^18 values the packing pass finds the true maximum: any value anywhere keeps its bits, from the first to the last
+    element, aligned or not; beside it the ordinary values keep those of fp32 sums."""
+    from tdc_b200 import tc
+    kind, R, stride, _ = KINDS[{0: "3x3", 1: "3x3s2", 2: "7x7s2", 3: "rows"}[pack]]
+    if pack >= 2:
+        C = min(C, 5)
+    x0, w, scale, bias = draw(31, B, C, 24, H, W, R)
+    room = torch.empty(x0.numel() + 1, device="cuda")
+    for at, off in ((0, 0), (x0.numel() - 1, 1), (x0.numel() // 2 + 1, 0)):
+        x = room[off:off + x0.numel()].view_as(x0).copy_(x0)
+        x.view(-1)[at] = 1e7
+        net = N.Net(B, C, H, W, x.device)
+        net.conv(net.pack(pack), kind, w, scale, bias, True, out=N.NCHW)
+        ref = conv64(x, w, stride, scale, bias, True)
+        y = net.finish(ref.shape)(x)
+        assert rel(y, ref) <= FP32_TOL and tc.status() == 0
+        away = (F.conv2d((x == 1e7).double(), torch.ones(24, C, R, R, device="cuda").double(), None, stride, R // 2) == 0).double()
+        assert float(((y - ref) * away).abs().max()) <= FP32_TOL * max(1.0, float((ref * away).abs().max()))
+
+
+@pytest.mark.parametrize("B,C,R1,H,stride", [(1, 64, 32, 14, 1), (1, 64, 32, 14, 2), (2, 512, 8, 32, 1), (2, 512, 8, 32, 2)])
+def test_auto_modules_take_any_value_where_they_began_in_fp32(N, B, C, R1, H, stride):
+    """Layers below the size from which "auto" used tensor cores have no range: small inputs are packed with their true one, larger ones
+    are not packed."""
+    import tdc_b200 as T
+    from tdc_b200 import dispatch, tc
+
+    class HP:
+        ranks = {"l": [32, R1]}
+    torch.manual_seed(7)
+    m = T.TKConv2dC_B200(C, 64, 3, stride=stride, padding=1, bias=False, hp_dict=HP, name="l").cuda()
+    m.precision = "auto"
+    x = torch.randn(B, C, H, H, device="cuda")
+    assert not dispatch._on_tensor_cores(B, C, R1, H, H, 1, 1, 1, 0)
+    x[-1, 1, 3, 5] = 1e6
+    ref = F.conv2d(F.conv2d(F.conv2d(x.double(), m.first_kernel.double()), m.core_kernel.double(), None, stride, 1), m.last_kernel.double())
+    with torch.no_grad():
+        assert rel(m(x), ref) <= FP32_TOL and tc.status() == 0
