@@ -552,13 +552,14 @@ def main():
         w = torch.randn(R2, R1, 3, 3, generator=g) * (2.0 / (R2 * 9)) ** 0.5
         xd, wk = x.to(dev), w.to(dev)
         layers.append(dict(H=H, R1=R1, R2=R2, x=xd, w=T.permute_weights(wk), wk=wk, y=torch.empty(BATCH, R2, H, H, device=dev),
-                           tile=T.best_tile(BATCH, R1, H, H, R2, 3, 3, 1, 1), tc4=T.TcConv(wk, mode=4), tc3=T.TcConv(wk, mode=3), tc1=T.TcConv(wk, mode=1),
+                           tc4=T.TcConv(wk, mode=4), tc3=T.TcConv(wk, mode=3), tc1=T.TcConv(wk, mode=1),
                            x_host=x, w_host=w))
 
     # The step the headline is quoted on: every layer on the fastest path that keeps fp32-level
     # results (1e-5 bar) — at batch 64 that is the tensor-core kernel with operands split into two
-    # fp16 parts (3xFP16) for all eight shapes (one launch each; the kernel takes the scale that
-    # brings the input into fp16's range from a sample of the input).  Split TF32
+    # fp16 parts (3xFP16) for all eight shapes (one launch each, or a packing launch and one on packed
+    # operands where that is faster; the scale that brings the input into fp16's range comes from
+    # a sample of the input).  Split TF32
     # parts, the fp32 FMA kernels and plain TF32 are timed beside it below.
     def step_one_stream():
         for L in layers:
@@ -586,7 +587,7 @@ def main():
 
     def step_simt():
         for L in layers:
-            T.core_conv2d(L["x"], L["w"], 1, 1, w_layout=T.W_CRSK, tile=L["tile"], out=L["y"])
+            T.core_conv2d(L["x"], L["w"], 1, 1, w_layout=T.W_CRSK, out=L["y"])
 
     def barrier():
         if dist is not None:
@@ -648,13 +649,12 @@ def main():
         row = dict(H=L["H"], R1=L["R1"], R2=L["R2"], B=BATCH)
         for name, fn in (("tc4", lambda L=L: L["tc4"](L["x"], out=L["y"])), ("tc3", lambda L=L: L["tc3"](L["x"], out=L["y"])),
                          ("tc1", lambda L=L: L["tc1"](L["x"], out=L["y"])),
-                         ("simt", lambda L=L: T.core_conv2d(L["x"], L["w"], 1, 1, w_layout=T.W_CRSK, tile=L["tile"], out=L["y"]))):
+                         ("simt", lambda L=L: T.core_conv2d(L["x"], L["w"], 1, 1, w_layout=T.W_CRSK, out=L["y"]))):
             us = time_layer(fn)
             row[name + "_us"] = us
             row[name + "_tflops"] = fl / us / 1e6
             row[name + "_rel_err_fp64"] = float((L["y"][:2].double() - ref).abs().max() / ref.abs().max())
         row["gbs_tc4"] = by / row["tc4_us"] / 1e3
-        row["tile_simt"] = list(L["tile"].as_tuple())
         per_layer.append(row)
     tot_fl = sum(conv_flops(BATCH, r["H"], r["R1"], r["R2"]) for r in per_layer)
     tot_by = sum(conv_bytes(BATCH, r["H"], r["R1"], r["R2"]) for r in per_layer)
@@ -672,7 +672,7 @@ def main():
                          "algorithmic_bytes": conv_bytes(BATCH, dom["H"], dom["R1"], dom["R2"]),
                          "source": "recorded: dram__bytes_read.sum + dram__bytes_write.sum of the dominant launch in an earlier ncu "
                                    "capture of this command (not measured by this run)"},
-        "kernel": "conv_tc_persist_kernel (tcgen05 kind::f16, operands split into two fp16 parts), the 8 launches of a step, L2 flushed before each",
+        "kernel": "conv_tc_persist_kernel, or pack_kernel and a conv_pk kernel (tcgen05 kind::f16, operands split into two fp16 parts), the 8 layers of a step, L2 flushed before each",
         "peak_source": "algorithmic FLOPs against bf16_tflops/3: the measured cuBLAS bf16 rate of MEASURED_PEAKS.json (%s) as the dense "
                        "fp16 rate, divided by the three fp16 products each fp32-level product costs" % peaks["source"],
         "dominant_launch": {k: dom[k] for k in ("H", "R1", "R2", "tc4_us", "tc4_tflops")},
@@ -688,13 +688,14 @@ def main():
         "value": len(SWEEP) * BATCH * world / (ms_simt * 1e-3), "unit": UNIT, "ms_per_step": ms_simt,
         "roofline": {"bound": "fp32", "achieved": tot_fl / tot_simt / 1e6, "peak": fp32_peak, "unit": "TFLOP/s",
                      "frac": tot_fl / tot_simt / 1e6 / fp32_peak,
-                     "kernel": "conv_f32_kernel (fp32 FMA, bit-reproducible), the 8 launches of a step",
+                     "kernel": "the fp32 kernels as a call without a tile takes them (conv_f32_gemm_kernel: FMA, bit-reproducible), the 8 launches of a step",
                      "peak_source": "SMs x 128 lanes x 2 x max SM clock from MEASURED_PEAKS.json (%s)" % peaks["source"]},
     }
     tf32 = {"value": len(SWEEP) * BATCH * world / (tot_tc1 * 1e-6), "unit": UNIT, "tolerance": 5e-3,
             "max_rel_err_fp64": max(r["tc1_rel_err_fp64"] for r in per_layer),
             "note": "plain TF32 (one MMA per product), from per-layer timings; reported separately from the fp32-level paths"}
 
+    launches = sum(2 if any(L["tc4"]._nets.values()) else 1 for L in layers)      # a layer in packed form: the packing pass and the convolution
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
         "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
@@ -708,7 +709,7 @@ def main():
                    "streams": "the eight independent layers of a step are issued alternately on two streams forked from and joined to "
                               "the timed stream (ms_per_step_one_stream: the same step on one stream)",
                    "parallelism": "batch shards, no collective" if world > 1 else "single GPU"},
-        "clocks": clocks, "gpu_launches": len(SWEEP) * args.steps, "roofline": roofline,
+        "clocks": clocks, "gpu_launches": launches * args.steps, "roofline": roofline,
         "us_per_layer_b64": ms_step * 1e3 / len(SWEEP), "ms_per_step_one_stream": ms_step_one,
         "fp32_fma_path": simt, "tf32_path": tf32, "tf32x3_path": {"value": len(SWEEP) * BATCH * world / (tot_tc3 * 1e-6), "unit": UNIT,
                                                                   "max_rel_err_fp64": max(r["tc3_rel_err_fp64"] for r in per_layer)},
@@ -829,9 +830,8 @@ def main():
             H, R1, R2 = L["H"], L["R1"], L["R2"]
             wk = L["wk"]
             x1 = L["x"][:1].contiguous()
-            t1 = T.best_tile(1, R1, H, H, R2, 3, 3, 1, 1)
             y1 = torch.empty(1, R2, H, H, device=dev)
-            us1_fp32 = time_layer(lambda: T.core_conv2d(x1, L["w"], 1, 1, w_layout=T.W_CRSK, tile=t1, out=y1), iters=20)
+            us1_fp32 = time_layer(lambda: T.core_conv2d(x1, L["w"], 1, 1, w_layout=T.W_CRSK, out=y1), iters=20)
             us1_tc4 = time_layer(lambda: L["tc4"](x1, out=y1), iters=20)
             # batch 1 as the dispatch rule runs it: tensor cores where the layer has the tiles and the arithmetic for it
             from tdc_b200 import tc as _tc
@@ -845,8 +845,7 @@ def main():
                               cudnn_us_b64=cud64, rel_err_fp64_b64=r64["tc4_rel_err_fp64"], cudnn_rel_err_fp64_b64=cud_err,
                               frac_b64=conv_flops(BATCH, H, R1, R2) / r64["tc4_us"] / 1e6 / (f16_peak / 3.0),
                               us_b1=us1, path_b1=b1_path, us_b1_fp32_fma=us1_fp32, us_b1_fp16x3=us1_tc4,
-                              frac_fp32_b1=conv_flops(1, H, R1, R2) / us1_fp32 / 1e6 / fp32_peak, cudnn_us_b1=cud1,
-                              tile_b1=list(t1.as_tuple())))
+                              frac_fp32_b1=conv_flops(1, H, R1, R2) / us1_fp32 / 1e6 / fp32_peak, cudnn_us_b1=cud1))
         line["layers"] = table
         # what the timing itself costs: a kernel that does nothing, between the same pair of events after the same flush
         one = torch.zeros(1, device=dev)
