@@ -68,12 +68,13 @@ GemmTile gemm_choose(const Shape& s) {
 
 // Measured against conv_f32_kernel on its table's (or model's) tile on 214 layers: 1.1 - 6 times as fast on all but 13.
 // Those have filters beyond 3x3, whose windows the rectangles of conv_f32_kernel read once where this kernel gathers every
-// row (with torch's filter layout this kernel wins all the same), or 33 - 40 output channels on large images, which fill
-// 64-channel tiles by little more than a half.
+// row (with torch's filter layout this kernel wins all the same), or one tile of 64 channels that their outputs fill to five
+// eighths at most (33 - 40 channels, above 4 GFLOP): the rectangles of conv_f32_kernel go in steps of 4 channels.
 bool gemm_wins(const Shape& s, bool channel_last) {
     if (!gemm_fits(s)) return false;
     if (s.R * s.S > 9) return !channel_last || s.C < 16;
-    return !(s.R == 3 && s.K > 32 && s.K <= 40 && 18.0 * s.C * s.K * s.B * s.Ho() * s.Wo() > 4e9);
+    const bool half_empty = s.K > 32 && s.K <= 64 * 5 / 8;
+    return !(s.R == 3 && half_empty && 18.0 * s.C * s.K * s.B * s.Ho() * s.Wo() > 4e9);
 }
 
 int gemm_launch(const ConvArgs& base, const Shape& s, const GemmTile& t, int device, cudaStream_t stream) {
