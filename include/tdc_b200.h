@@ -441,11 +441,13 @@ typedef struct tdc_net tdc_net;
 
 /* What tdc_net_pack, the first step of a net, makes of the NCHW input.  Its scale comes from the maxima a run is given, else from the true
  * maximum of an input of up to 2^18 values and from a sample of a larger one, with tdc_conv2d_tc_ranged's headroom of 256; a value
- * beyond makes outputs that are not finite and sets the status word to 2. */
+ * beyond makes outputs that are not finite and sets the status word to 2.  With TDC_NET_PACK_EXACT added a larger input's true maximum
+ * is found by a pass of its own (one more launch). */
 #define TDC_NET_PACK       0   /* channels and positions as they are */
 #define TDC_NET_PACK_SPLIT 1   /* positions by (row parity, column parity): what stride-2 convolutions read */
 #define TDC_NET_PACK_S2D   2   /* for TDC_NET_CONV7x7_S2 */
 #define TDC_NET_PACK_ROWS  3   /* for TDC_NET_CONV3x3_ROWS: few channels */
+#define TDC_NET_PACK_EXACT 0x100
 /* Convolution kinds ("same" padding). */
 #define TDC_NET_CONV1x1      0
 #define TDC_NET_CONV3x3      1

@@ -58,7 +58,7 @@ int opt_in(const void* fn, int smem_max) {
 }
 
 // A tdc_status; the steps that call other entry points return theirs.
-int launch(const void* fn, dim3 grid, int threads, int cluster, size_t smem, void* args, cudaStream_t st) {
+int launch_args(const void* fn, dim3 grid, int threads, int cluster, size_t smem, void** argv, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -67,9 +67,12 @@ int launch(const void* fn, dim3 grid, int threads, int cluster, size_t smem, voi
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
-    void* argv[] = {args};
     const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, argv);
     return e == cudaSuccess ? TDC_OK : fail(TDC_ERR_CUDA, "launch: %s", cudaGetErrorString(e));
+}
+int launch(const void* fn, dim3 grid, int threads, int cluster, size_t smem, void* args, cudaStream_t st) {
+    void* argv[] = {args};
+    return launch_args(fn, grid, threads, cluster, smem, argv, st);
 }
 
 struct Buffer { size_t bytes = 0, off = 0; int def = -1, last = -1; };
@@ -256,6 +259,8 @@ void tdc_net_destroy(tdc_net* n) { delete n; }
 
 int tdc_net_pack(tdc_net* n, int kind, int* out) {
     if (!n || !out) return fail(TDC_ERR_NULL, "net and out must be non-NULL");
+    const bool want_exact = kind & TDC_NET_PACK_EXACT;
+    kind &= ~TDC_NET_PACK_EXACT;
     if (kind < PACK_SAME || kind > PACK_ROW3) return fail(TDC_ERR_UNSUPPORTED, "pack kind %d", kind);
     if (!n->tensors.empty()) return fail(TDC_ERR_UNSUPPORTED, "packing the input is a net's first step");
     Space s;
@@ -269,17 +274,34 @@ int tdc_net_pack(tdc_net* n, int kind, int* out) {
     PackArgs a{};
     a.B = n->B; a.C = n->C; a.H = n->H; a.W = n->W;
     a.groups = t.groups; a.front = space_front(s); a.d = s; a.y_plane = tdc_net::pk_plane(t); a.status = n->f.status;
-    const bool exact = (long long)n->B * n->C * n->H * n->W <= PACK_EXACT;
+    const long long values = (long long)n->B * n->C * n->H * n->W;
+    const bool exact = values <= PACK_EXACT;
+    a.sample_step = (uint32_t)((values + 3 * OPS_THREADS - 1) / (3 * OPS_THREADS));
     unsigned grid = blocks_for(items, n->f);
     if (exact) grid = std::min<unsigned>((grid + PACK_CLUSTER - 1) / PACK_CLUSTER, PACK_SLOTS / PACK_CLUSTER) * PACK_CLUSTER;
     t.slots = (int)grid;
     const void* const forms[2][4] = {{(const void*)&pack_kernel<PACK_SAME, false>, (const void*)&pack_kernel<PACK_SPLIT, false>, (const void*)&pack_kernel<PACK_S2D, false>, (const void*)&pack_kernel<PACK_ROW3, false>},
                                      {(const void*)&pack_kernel<PACK_SAME, true>, (const void*)&pack_kernel<PACK_SPLIT, true>, (const void*)&pack_kernel<PACK_S2D, true>, (const void*)&pack_kernel<PACK_ROW3, true>}};
     const void* fn = forms[exact][kind];
-    n->ops.push_back([n, id, a, grid, fn, exact](const RunArgs& r) {
+    const int range = want_exact && !exact ? n->buffer(sizeof(float) * tdc_tc::ABSMAX_SLOTS) : -1;
+    if (range >= 0) {
+        const unsigned blocks = (unsigned)std::min<long long>((values / 4 + OPS_THREADS - 1) / OPS_THREADS, 2ll * n->f.sms < tdc_tc::ABSMAX_SLOTS ? 2ll * n->f.sms : tdc_tc::ABSMAX_SLOTS);
+        n->ops.push_back([n, range, values, blocks](const RunArgs& r) {
+            if (r.x_absmax) return (int)TDC_OK;
+            const float* x = r.x;
+            float* slots = reinterpret_cast<float*>(r.arena + n->buffers[range].off);
+            long long count = values;
+            int n_slots = tdc_tc::ABSMAX_SLOTS;
+            void* argv[] = {&x, &count, &slots, &n_slots};
+            return launch_args((const void*)&range_kernel, dim3(blocks), OPS_THREADS, 1, 0, argv, r.st);
+        });
+        n->use(range);
+        n->use(t.pk);
+    }
+    n->ops.push_back([n, id, a, grid, fn, exact, range](const RunArgs& r) {
         PackArgs p = a;
         const Tensor& t = n->tensors[id];
-        p.x = r.x; p.absmax = r.x_absmax; p.absmax_n = tdc_tc::ABSMAX_SLOTS;
+        p.x = r.x; p.absmax = r.x_absmax || range < 0 ? r.x_absmax : reinterpret_cast<const float*>(r.arena + n->buffers[range].off); p.absmax_n = tdc_tc::ABSMAX_SLOTS;
         p.y = n->pk_at(r, t);
         p.y_scale = n->meta_at(r, t); p.y_slots = p.y_scale + 1;
         p.zero = p.y_slots + PACK_SLOTS; p.zeros = (int)n->meta_floats - (1 + PACK_SLOTS);

@@ -39,6 +39,7 @@ struct PackArgs {
     float* y_scale; float* y_slots;       // the partial maxima of what it wrote, one per block
     float* zero; int zeros;               // the other tensors' meta blocks, cleared here (this is the first launch of a run)
     int* status;                          // 2 where a value does not fit
+    uint32_t sample_step;                 // a 1536th of x, rounded up: one value of each such piece is sampled
 };
 
 // NCHW -> packed planes.
@@ -49,7 +50,7 @@ struct PackArgs {
 //          block where the plain form takes nine taps of a block that is mostly zeros.
 // Bound by memory: 4 bytes read and 4 written per value.
 //
-// EXACT: launched in clusters of PACK_CLUSTER, each of which finds the true maximum of x for itself, every CTA of a share of it;
+// EXACT: the sample's place is taken by the true maximum.  Launched in clusters of PACK_CLUSTER, each of which finds the true maximum of x for itself, every CTA of a share of it;
 // the second reading comes out of cache.  For inputs of up to PACK_EXACT values that costs about what the round trip of the sample does,
 // and layers of that size ran on fp32 arithmetic, which has no range, before they ran on packed operands.
 constexpr int PACK_CLUSTER = 8;
@@ -86,6 +87,31 @@ __device__ __forceinline__ unsigned int cluster_absmax(const float* x, long long
     return m;
 }
 
+// The partial maxima of x, in the form a caller would give them: for larger inputs that want the true one (the clusters' readings add
+// up: at a million values they would cost 15 us, this pass costs one launch and one reading).
+__global__ void __launch_bounds__(OPS_THREADS) range_kernel(const float* x, long long n, float* slots, int n_slots) {
+    __shared__ unsigned int word;
+    pdl_enter();
+    unsigned int m = 0;
+    const long long step = (long long)gridDim.x * OPS_THREADS;
+    long long i = (long long)blockIdx.x * OPS_THREADS + threadIdx.x;
+    if (reinterpret_cast<uintptr_t>(x) % 16 == 0) {
+        const long long n4 = n / 4;
+#pragma unroll 4
+        for (; i < n4; i += step) {
+            const float4 v = reinterpret_cast<const float4*>(x)[i];
+            m = max(max(m, __float_as_uint(v.x) & 0x7fffffffu), __float_as_uint(v.y) & 0x7fffffffu);
+            m = max(max(m, __float_as_uint(v.z) & 0x7fffffffu), __float_as_uint(v.w) & 0x7fffffffu);
+        }
+        i = 4 * n4 + (long long)blockIdx.x * OPS_THREADS + threadIdx.x;
+    }
+    for (; i < n; i += step) m = max(m, __float_as_uint(x[i]) & 0x7fffffffu);
+    m = block_max(m, &word);
+    if (threadIdx.x == 0) slots[blockIdx.x] = __uint_as_float(m);
+    if (blockIdx.x == 0)
+        for (int k = (int)gridDim.x + threadIdx.x; k < n_slots; k += OPS_THREADS) slots[k] = 0.f;
+}
+
 template <int KIND, bool EXACT>
 __global__ void __launch_bounds__(OPS_THREADS, 2) pack_kernel(const PackArgs a) {
     __shared__ unsigned int word, peers[PACK_CLUSTER];
@@ -93,18 +119,17 @@ __global__ void __launch_bounds__(OPS_THREADS, 2) pack_kernel(const PackArgs a) 
     // the power of two the values are stored at: from the given maxima, the true one, or from 1536 values spread over x, which leaves a
     // factor of 256 for what the sample missed (what lies beyond is reported: the true maximum is known at the end, and the
     // convolution's outputs are NaN).  One value of each 1536th of x, at an offset that goes round by the golden ratio: at a fixed
-    // offset a batch of 16 images of 3 x 224 x 224 was sampled in one column.
+    // one a batch of 16 images of 3 x 224 x 224 was sampled in one column.
     const long long n = (long long)a.B * a.C * a.H * a.W;
     unsigned int m = 0;
     if (a.absmax) m = slots_max(a.absmax, a.absmax_n, threadIdx.x, OPS_THREADS);
     else if (EXACT) m = cluster_absmax(a.x, n, &word, peers);
     else {
-        constexpr unsigned long long PARTS = 3 * OPS_THREADS;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const unsigned long long j = threadIdx.x + i * OPS_THREADS, lo = j * (unsigned long long)n / PARTS, hi = (j + 1) * (unsigned long long)n / PARTS;
-            const unsigned long long k = lo + __umul64hi((unsigned long long)((uint32_t)j * 2654435769u) << 32, hi - lo);      // in [lo, hi), or lo < n
-            m = max(m, __float_as_uint(a.x[k]) & 0x7fffffffu);
+            const uint32_t j = threadIdx.x + i * OPS_THREADS;
+            const unsigned long long k = (unsigned long long)j * a.sample_step + __umulhi(j * 2654435769u, a.sample_step);
+            if (k < (unsigned long long)n) m = max(m, __float_as_uint(a.x[k]) & 0x7fffffffu);
         }
     }
     const float s = range_scale(__uint_as_float(block_max(m, &word)), a.absmax || EXACT ? 14 : 8);

@@ -15,6 +15,7 @@ from ._lib import ERR_SHAPE, NetConv, NetNchw, NetPool, TdcError, check, lib
 from .ops import _dev_f32, _on_device, _stream
 
 PACK, PACK_SPLIT, PACK_S2D, PACK_ROWS = range(4)
+PACK_EXACT = 0x100
 CONV1x1, CONV3x3, CONV3x3_S2, CONV7x7_S2, CONV3x3_ROWS, CONV1x1_S2 = range(6)
 PACKED, PLANES, NCHW = 1, 2, 4
 
@@ -99,9 +100,10 @@ class Net:
             lib.tdc_net_destroy(self._h)
             self._h = None
 
-    def pack(self, kind=PACK):
+    def pack(self, kind=PACK, exact=False):
+        """`exact`: the true maximum of an input of any size (of up to 2^18 values it is found anyway)."""
         out = C.c_int()
-        check(lib.tdc_net_pack(self._h, kind, C.byref(out)))
+        check(lib.tdc_net_pack(self._h, kind | (PACK_EXACT if exact else 0), C.byref(out)))
         return self._made(out.value, self.shape[1] * {PACK_S2D: 4, PACK_ROWS: 3}.get(kind, 1))
 
     def _made(self, tensor, channels):

@@ -173,18 +173,19 @@ ABSMAX_FLOATS = 1024      # TDC_TC_ABSMAX_FLOATS
 
 
 def leave_range(y, absmax):
-    """Keeps on y the partial maxima of |y| that its kernel wrote, for the convolution that reads y next."""
-    y._tdc_absmax, y._tdc_absmax_at = absmax, None if y.is_inference() else y._version
+    """Keeps on y the partial maxima of |y| that its kernel wrote, for the convolution that reads y next.  (A new tensor, which was never
+    written to, needs the first attribute only.)"""
+    y._tdc_absmax = absmax
+    if not y.is_inference():
+        y._tdc_absmax_at = y._version
 
 
 def range_of(x):
     """The partial maxima kept on x, or None: there are none, or x was written to since."""
-    d = x.__dict__
-    hit = d.get("_tdc_absmax")
-    if hit is None:
-        return None
-    at = d.get("_tdc_absmax_at")
-    return hit if at is None or at == x._version else None
+    hit = x.__dict__.get("_tdc_absmax")
+    if hit is None or x.is_inference() or x._version == x.__dict__.get("_tdc_absmax_at", 0):
+        return hit
+    return None
 
 
 POOL_MAX, POOL_AVG_INCLUDE_PAD, POOL_AVG_EXCLUDE_PAD = 0, 1, 2

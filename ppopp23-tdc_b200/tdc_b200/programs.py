@@ -19,7 +19,7 @@ from torch.nn.modules import module as _module
 
 from . import net as N
 from ._lib import ERR_SHAPE, ERR_SMEM, ERR_UNSUPPORTED, NetConv, TdcError, check, lib
-from .ops import ABSMAX_FLOATS, _stream, leave_range, range_of
+from .ops import ABSMAX_FLOATS, _stream, range_of
 
 import ctypes as C
 
@@ -609,18 +609,19 @@ class _LayerNet:
 
 def layer(module, x):
     """A Tucker module's output for a contiguous fp32 x through its net, or None where it has to run step by step."""
-    p = module._parameters
+    d = module.__dict__
+    p = d["_parameters"]
     first, core, last, bias = p.get("first_kernel"), p.get("core_kernel"), p.get("last_kernel"), p.get("bias")
     if first is None or core is None or last is None:      # parametrised or pruned: they are made anew on every access
         return None
     mark = (first._version, first.data_ptr(), core._version, core.data_ptr(), last._version, last.data_ptr(),
-            None if bias is None else (bias._version, bias.data_ptr()))
-    cache = module.__dict__.get("_layer_net")
+            None if bias is None else (bias._version, bias.data_ptr()), d["stride"], d["padding"], d["dilation"], d["groups"])
+    cache = d.get("_layer_net")
     if cache is None or cache.mark != mark:
-        cache = module.__dict__["_layer_net"] = _LayerNet()
+        cache = d["_layer_net"] = _LayerNet()
         cache.mark = mark
         cache.keep = [t.detach() for t in (first, core, last, bias) if t is not None]      # the mark holds their addresses
-    key = (x.shape, module.precision, x.device.index, module.stride, module.padding, module.dilation, module.groups)
+    key = (x.shape, module.precision, x.device.index)
     net = cache.nets.get(key)
     if net is None:
         N.make_room(cache.nets, _LayerNet.MOST)
@@ -628,12 +629,13 @@ def layer(module, x):
             net = cache.nets[key] = _build_layer(module, x)
     if not net:
         return None
+    # (from module to module, and from and to TcConv, the exact range: only the first of a chain looks at its input)
+    xmax = range_of(x) if "_tdc_absmax" in x.__dict__ else None
     if not net.leaves_range:
-        return net(x, None, range_of(x))
-    # (from module to module, and from and to TcConv, the exact range: only the first of a chain samples)
+        return net(x, None, xmax)
     ymax = x.new_empty(ABSMAX_FLOATS)
-    y = net(x, None, range_of(x), ymax)
-    leave_range(y, ymax)
+    y = net(x, None, xmax, ymax)
+    y._tdc_absmax = ymax
     return y
 
 
@@ -654,19 +656,23 @@ def _one_launch_wins(module, x):
     return direct <= max(13.3, packed)          # (the host time of a call that packs: TcConv._packs)
 
 
-EXACT_RANGE = 1 << 18      # values up to which packing finds the true maximum (csrc/pk_ops.cuh: PACK_EXACT); above, it samples
-
-
-def _has_no_range(module, x):
-    """A module whose layer-by-layer form begins in fp32 arithmetic takes any input; on packed operands that holds where the true maximum
-    is found."""
+def _began_in_fp32(module, x):
+    """Whether the layer-by-layer form of a module under "auto" begins in fp32 arithmetic, which takes any input: on packed operands that
+    wants the true maximum.  (Where it begins on tensor cores it samples, and so does packing.)"""
     from . import dispatch as D
     B, Cc, H, W = x.shape
-    if x.numel() <= EXACT_RANGE:
-        return False
     if D.tucker_strategy(module, x, "auto") == "dense":
         return not D._on_tensor_cores(B, Cc, module.out_channels, H, W, 3, 3, module.stride[0], 1)
     return not D._on_tensor_cores(B, Cc, module.in_rank, H, W, 1, 1, 1, 0)
+
+
+def _ended_in_fp32(module, x, Ho, Wo):
+    """Likewise its end, which then leaves no range; small calls are over sooner than the table for one is allocated."""
+    from . import dispatch as D
+    B, Cc, H, W = x.shape
+    if D.tucker_strategy(module, x, "auto") == "dense":
+        return _began_in_fp32(module, x)
+    return not D._on_tensor_cores(B, module.out_rank, module.out_channels, Ho, Wo, 1, 1, 1, 0)
 
 
 def _build_layer(module, x):
@@ -688,12 +694,11 @@ def _build_layer(module, x):
         stride = _square(module, 3)
         net = N.Net(B, Cc, H, W, x.device)
         K, shape = module.out_channels, (B, module.out_channels, -(-H // stride), -(-W // stride))
-        unpacked = module.precision == "auto" and (_has_no_range(module, x) or (stride == 1 and _one_launch_wins(module, x)))
-        if unpacked and stride == 2:
-            return False
-        if not unpacked:
-            at = At(net.pack(N.PACK_SPLIT if stride == 2 else N.PACK), Cc, H, W, stride == 2)
+        auto = module.precision == "auto"
+        if not (auto and stride == 1 and _one_launch_wins(module, x)):
+            at = At(net.pack(N.PACK_SPLIT if stride == 2 else N.PACK, auto and _began_in_fp32(module, x)), Cc, H, W, stride == 2)
             conv(net, module, at, None, None, False, module.precision, out=N.NCHW)
+            net.leaves_range = not (auto and _ended_in_fp32(module, x, *shape[2:]))
             return net.finish(shape)
 
         # the launches of the layer-by-layer path (dispatch.one_conv under "auto"), made from native code

@@ -184,7 +184,7 @@ class TcConv:
             if net is not None:
                 ymax = x.new_empty(ABSMAX_FLOATS)
                 out = x.new_empty(net.out_shape)
-                xmax = range_of(x)
+                xmax = range_of(x) if "_tdc_absmax" in x.__dict__ else None
                 arena = x.new_empty(net.arena_floats)
                 stream = _stream()
                 if stream not in net._streams:
@@ -193,7 +193,7 @@ class TcConv:
                                        net.arena_bytes, stream)
                 if code:
                     _check(code)
-                leave_range(out, ymax)
+                out._tdc_absmax = ymax
                 return out
             B, _, H, W = x.shape
             out = x.new_empty(rec[5])
@@ -201,10 +201,10 @@ class TcConv:
                 code = lib.tdc_conv2d_tc(plan, x.data_ptr(), wt.data_ptr(), out.data_ptr(), B, H, W, None, flags, _stream())
             else:
                 ymax = x.new_empty(ABSMAX_FLOATS)
-                xmax = range_of(x)
+                xmax = range_of(x) if "_tdc_absmax" in x.__dict__ else None
                 code = lib.tdc_conv2d_tc_ranged(plan, x.data_ptr(), wt.data_ptr(), out.data_ptr(), B, H, W, None, flags,
                                                 xmax.data_ptr() if xmax is not None else None, ymax.data_ptr(), _stream())
-                leave_range(out, ymax)
+                out._tdc_absmax = ymax
             if code:
                 _check(code)
             return out

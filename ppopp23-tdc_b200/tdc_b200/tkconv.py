@@ -160,7 +160,7 @@ class TKConv2dC_B200(nn.Module):
                 return y
         if square and self.precision != "fp32":
             # each of the three steps on the kernel that suits it (tensor cores where a plan exists and, under
-            # "auto", the step is large enough; the fp32 FMA kernel with its table tile otherwise)
+            # "auto", the step is large enough; the fp32 FMA kernels otherwise)
             from .dispatch import one_conv, tucker_strategy
             p = self.precision
             bias = None if self.bias is None else self.bias.detach()

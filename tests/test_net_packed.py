@@ -526,7 +526,7 @@ def test_small_inputs_have_their_true_range(N, pack, B, C, H, W):
 @pytest.mark.parametrize("B,C,R1,H,stride", [(1, 64, 32, 14, 1), (1, 64, 32, 14, 2), (2, 512, 8, 32, 1), (2, 512, 8, 32, 2)])
 def test_auto_modules_take_any_value_where_they_began_in_fp32(N, B, C, R1, H, stride):
     """Layers below the size from which "auto" used tensor cores have no range: small inputs are packed with their true one, larger ones
-    are not packed."""
+    after a pass that finds it."""
     import tdc_b200 as T
     from tdc_b200 import dispatch, tc
 
