@@ -48,6 +48,7 @@ def channel_last(owner, name, w):
     hit = store.get(name)
     if hit is None or hit[0] != key:
         with building(w.device):
+            building.made()
             w = w.detach().contiguous()
             hit = store[name] = (key, ops.permute_weights(w), w)      # (the filter itself too: its address is the key)
     return hit[1]

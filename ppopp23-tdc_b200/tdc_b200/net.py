@@ -38,7 +38,8 @@ class building:
     """`with building(device):` around work whose results are kept — prepared filters, folded BatchNorms, channel-last copies.  They
     are shared between nets, and the next net may be built by another thread on another stream: one is built at a time,
     and its stream first waits for the work of the one before."""
-    _lock, _depth, _last = threading.RLock(), 0, {}
+    _lock, _depth, _nets, _made = threading.RLock(), 0, [], False
+    _last = {}          # device -> (the event behind the last such work, the stream it was put on)
 
     def __init__(self, device):
         self.device, self.on = device, _on_device(device)
@@ -47,18 +48,33 @@ class building:
         building._lock.acquire()
         building._depth += 1
         self.on.__enter__()
-        last = building._last.get(self.device.index) if building._depth == 1 else None
-        if last is not None and not torch.cuda.is_current_stream_capturing():
-            torch.cuda.current_stream().wait_event(last)
+        if building._depth > 1:
+            building._made = True
+            return
+        building._made = False
+        last = building._last.get(self.device.index)
+        if last is not None and last[1] != _stream() and not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream().wait_event(last[0])
 
     def __exit__(self, *exc):
         try:
             if building._depth == 1:
-                building._last[self.device.index] = _mark(self.device) or building._last.get(self.device.index)
+                if building._made:
+                    event = _mark(self.device)
+                    if event is not None:
+                        building._last[self.device.index] = (event, _stream())
+                for net in building._nets:
+                    net._event, net._built_on = building._last.get(self.device.index, (None, None))
+                building._nets.clear()
         finally:
             building._depth -= 1
             self.on.__exit__(*exc)
             building._lock.release()
+
+    @staticmethod
+    def made():
+        """Says that something was prepared (without it a build leaves no event: it only read what was there)."""
+        building._made = True
 
 
 def make_room(table, most):
@@ -88,7 +104,7 @@ class Net:
         self._h = C.c_void_p()
         self._keep = []                 # everything the launches point to
         self._channels = {-1: Cc}       # tensor -> its channels (-1: the input)
-        self._event, self._streams = None, set()
+        self._event, self._built_on, self._streams = None, None, set()
         self.leaves_range = False       # a run writes the partial maxima of |y| it is given room for
         self.nchw, self.features = False, False      # which steps the network builders take, and whether they end at the classifier (programs.py)
         self.clocks = 0.0
@@ -147,6 +163,7 @@ class Net:
         at, key = (name, kind, nt, scale is None, bias is None), _key(weight, scale, bias)
         hit = store.get(at)
         if hit is None or hit[0] != key:
+            building.made()
             w = weight.detach()
             buf = torch.empty(nbytes, dtype=torch.uint8, device=w.device)
             check(lib.tdc_net_filter_prepare(kind, w.shape[0], w.shape[1], nt, _dev_f32(w, "weight"), scale.data_ptr() if scale is not None else None,
@@ -225,7 +242,10 @@ class Net:
         check(lib.tdc_net_finish(self._h, C.byref(n)))
         self.arena_bytes, self.out_shape = n.value, tuple(out_shape)
         self.arena_floats = max(1, -(-n.value // 4))
-        self._event = _mark(self.device)
+        if building._lock._is_owned():
+            building._nets.append(self)             # (its event: the end of the build, before anyone is handed the net)
+        else:
+            self._event = _mark(self.device)
         return self
 
     def meet(self, stream):
@@ -234,7 +254,7 @@ class Net:
         if torch.cuda.is_current_stream_capturing():      # (captures begin on an idle device; what a graph reads is for its owner to keep)
             return
         current = torch.cuda.current_stream()
-        if self._event is not None:
+        if self._event is not None and stream != self._built_on:
             current.wait_event(self._event)
         for t in self._keep:
             if t is not None and t.is_cuda:

@@ -57,6 +57,7 @@ def fold_bn(bn):
         buf = torch.empty(2 * n4 + 2, device=dev, dtype=torch.float32)
         scale, shift, bound = buf[:n], buf[n4:n4 + n], buf[2 * n4:]
         with N.building(dev):
+            N.building.made()
             if all(t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.device == dev and t.numel() == n) for t in tensors):
                 var, mean, g, b = (None if t is None else t.data_ptr() for t in tensors)
                 check(lib.tdc_net_fold_bn(var, mean, g, b, bn.eps, n, scale.data_ptr(), shift.data_ptr(), bound.data_ptr(), _stream()))
@@ -136,6 +137,7 @@ def _with_bias(conv, scale, shift):
     kept = conv.__dict__.setdefault("_tdc_shift", N.Cache())
     hit = kept.get("shift")
     if hit is None or hit[0] != key:
+        N.building.made()
         b = conv.bias.detach() if scale is None else conv.bias.detach() * scale
         hit = kept["shift"] = (key, b if shift is None else shift + b, conv.bias.detach(), scale, shift)
     return hit[1]
@@ -568,11 +570,13 @@ def forward(model, x, build, head):
                 return None
             return y if native else head(y)
         else:
-            with cache.lock, N.building(x.device):
+            with cache.lock:
                 if key not in cache.nets:
+                    with N.building(x.device):
+                        built = _build(model, x, build, head, native is None)
                     N.make_room(cache.nets, Nets.MOST)
                     cache.classifier = native or cache.classifier
-                    cache.nets[key] = _build(model, x, build, head, native is None)
+                    cache.nets[key] = built
     return None
 
 
@@ -624,9 +628,10 @@ def layer(module, x):
     key = (x.shape, module.precision, x.device.index)
     net = cache.nets.get(key)
     if net is None:
-        N.make_room(cache.nets, _LayerNet.MOST)
         with N.building(x.device):
-            net = cache.nets[key] = _build_layer(module, x)
+            net = _build_layer(module, x)
+        N.make_room(cache.nets, _LayerNet.MOST)
+        cache.nets[key] = net
     if not net:
         return None
     # (from module to module, and from and to TcConv, the exact range: only the first of a chain looks at its input)

@@ -313,6 +313,7 @@ def cached(owner, name, weight, mode, w_layout=_lib.W_KCRS, general=False):
     hit = store.get((name, mode, w_layout, general))
     if hit is None or hit[0] != key:
         with building(weight.device):
+            building.made()
             hit = store[(name, mode, w_layout, general)] = (key, TcConv(weight.detach(), mode, w_layout, general, unbiased=True, snapshot=False))
     return hit[1]
 
