@@ -193,8 +193,8 @@ class TKResNet(nn.Module):
         self.set_precision(precision)
 
     def set_precision(self, precision):
-        """"fp32" (default): every conv on the fp32 FMA kernels; "auto": large layers on tensor cores
-        with split operands (fp32-level results), small ones on the fp32 kernels; "tf32": every
+        """"fp32" (default): every conv on the fp32 FMA kernels; "auto": tensor cores with split fp16
+        operands on packed activations (fp32-level results; layer by layer, small layers run on the fp32 kernels); "tf32": every
         conv with a tensor-core plan on tensor cores; "tf32x3" likewise, where that is the faster way to
         its fp32-level results."""
         if precision not in ("fp32", "auto", "fp16x3", "tf32x3", "tf32"):

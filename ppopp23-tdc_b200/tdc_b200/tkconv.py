@@ -24,7 +24,8 @@ class TKConv2dC_B200(nn.Module):
     # "fp16x3" / "tf32x3": tensor cores with operands split into two fp16 / TF32 parts, fp32-level results (1e-5 bar;
     #     fp16 parts need |x| and |w| within fp16's range of 65504);
     # "tf32": tensor cores, plain TF32 (5e-3 bar);
-    # "auto": split operands where the layer is large enough to fill the GPU, fp32 otherwise.
+    # "auto": split fp16 operands, packed or split as the launch goes, whichever form is estimated the fastest; steps too small for the
+    #     one-launch kernels run in fp32 where the module is not packed.
     precision = "fp32"
 
     def __init__(self, in_channels: int, out_channels: int, kernel_size, stride=1, padding=0, dilation=1,
